@@ -214,6 +214,7 @@ int setup(md200_engine *e) {
   const size_t nt = static_cast<size_t>(B) * T;
   if (own_alloc(e, &d.mL, B) || own_alloc(e, &d.mwater, B) || own_alloc(e, &d.mstate, B) ||
       own_alloc(e, &d.mlo, B) || own_alloc(e, &d.mhi, B) || own_alloc(e, &d.malpha, B) ||
+      own_alloc(e, &d.mstart, B) ||
       own_alloc(e, &d.mtail, 2 * static_cast<size_t>(B)) || own_alloc(e, &d.tail, 2 * nt) ||
       own_alloc(e, &d.layer64, static_cast<size_t>(B) * ROWS * d.Ls) ||
       own_alloc(e, &d.layer32, static_cast<size_t>(B) * ROWS * d.Ls) ||
@@ -226,7 +227,6 @@ int setup(md200_engine *e) {
       own_alloc(e, &d.trace_list, nt) || own_alloc(e, &d.repair_list, nt) ||
       own_alloc(e, &d.refine_list, 2 * nt * d.KB) ||
       own_alloc(e, &d.group_list, nt * nm) || own_alloc(e, &d.ctr, C_COUNT) ||
-      own_alloc(e, &d.gwin, nt * nm * 2) ||
       own_alloc(e, &e->d_stats, static_cast<size_t>(MD200_STAT_COUNT) * md200_engine::MAX_CHUNKS))
     return 1;
   // host-path device buffers

@@ -67,6 +67,7 @@ struct Dev {
   // prepared models
   int *mL, *mwater, *mstate;
   double *mlo, *mhi, *malpha;
+  int2 *mstart;     // first grid point and first seed a scan samples (no root lies below them)
   double *mtail;    // [B][2]: the two near-cutoff sample positions every scan that
                     // reaches the window end evaluates (hi, and vs_hs (1 - 1e-7))
   double4 *tail;    // [n_traces][2]: FP64 (c, F, g, log-magnitude) at those positions
@@ -99,7 +100,6 @@ struct Dev {
   int *olevels, *ocounts;
   double *grp;
   unsigned *gflags;
-  double *gwin;     // [B][nmodes][T][2]
   double *bounds_out;  // [B][2] windows used (optional)
   unsigned *pred;      // [B][T] prediction flags (optional)
   unsigned char *cflags;  // [B][T] continuity-screen flags (optional; FP32-scan runs)

@@ -147,8 +147,9 @@ __global__ void split_feed_fill(Dev d, int p) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < take; i += gridDim.x * blockDim.x) {
     const int t = d.trace_list[first + i];
     d.sp_act[p][base + i] = t;
-    d.sp_state[t] = scan_start(d, trace_ctx(d, t));
-    d.sp_kf[t] = 0;
+    const ScanState st = scan_start(d, trace_ctx(d, t));
+    d.sp_state[t] = st;
+    d.sp_kf[t] = max(0, static_cast<int>(st.gi) - 2);  // (as in the fused scan)
   }
 }
 
