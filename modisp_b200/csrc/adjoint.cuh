@@ -282,12 +282,12 @@ MD200_OUTLINE RowGrad love_layer_adjoint(const D2 &k, const D2 &w, double h, dou
 // Forward layer steps of the Jacobian sweeps (out of line).
 MD200_OUTLINE int rayleigh_step_k1(K1 e[5], const K1 &k, const K1 &k2, const K1 &w, const K1 &iw2, double h,
                                    double ivp, double vs2, double ivs, double rho, double irho) {
-  rayleigh_layer<K1, double>(e, k, k2, w, iw2, h, ivp, vs2, ivs, rho, irho);
+  rayleigh_layer_entries<K1, double>(e, k, k2, w, iw2, h, ivp, vs2, ivs, rho, irho);
   return scale_vector(e, 5, 1e-40);
 }
 MD200_OUTLINE void rayleigh_step_d2(D2 e[5], const D2 &k, const D2 &k2, const D2 &w, const D2 &iw2, double h,
                                     double ivp, double vs2, double ivs, double rho, double irho, double r) {
-  rayleigh_layer<D2, double>(e, k, k2, w, iw2, h, ivp, vs2, ivs, rho, irho);
+  rayleigh_layer_entries<D2, double>(e, k, k2, w, iw2, h, ivp, vs2, ivs, rho, irho);
   for (int i = 0; i < 5; ++i) e[i] = e[i] * r;
 }
 
