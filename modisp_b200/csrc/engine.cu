@@ -330,6 +330,9 @@ struct Ragged {
   const long long *outbase = nullptr;
 };
 
+// Runs of fewer traces list their brackets and roots as they come.
+constexpr int MODEL_LIST_MIN_TRACES = 4096;
+
 // Rounds of the split FP32 scan for a run of nt traces over an active set of
 // cap traces: enough for every trace of a typical run to finish (a trace takes
 // a round per SPLIT_SAMPLES samples, most take two or three); traces still
@@ -389,6 +392,7 @@ int enqueue(md200_engine *e, const double *h, const double *vp, const double *vs
     return fail("modisp_b200: group-velocity engine needs group output arrays");
   MD200_CK(cudaSetDevice(e->device));
   Dev d = e->d;
+  d.model_lists = 0;
   d.B = B;
   d.n_traces = rg.offsets ? rg.ntraces : B * e->T;
   d.ragged = rg.offsets ? 1 : 0;
@@ -448,25 +452,34 @@ int enqueue(md200_engine *e, const double *h, const double *vp, const double *vs
   MD200_CK(mark(2));
   // the split scan in auto mode: Rayleigh runs of SPLIT_MIN_TRACES traces or more
   // (the Love step is too cheap for the rounds to pay: measured slower)
+  // larger runs list their brackets and roots model by model (below a few thousand
+  // traces refinement is latency-bound and the extra launches cost what it gains)
+  Dev dm = d;
+  dm.model_lists = nt >= MODEL_LIST_MIN_TRACES ? 1 : 0;
+  const int model_blocks = (B + 3) / 4;
   const bool split = d.fp32 && (e->o.scan_mode == 2 ||
                                 (e->o.scan_mode == 0 && wave == 0 && nt >= SPLIT_MIN_TRACES));
   if (split) {
     const int rounds = split_rounds(nt, d.sp_cap);
-    const int launched = wave == 0 ? split_scan<0>(e, d, rounds, s) : split_scan<1>(e, d, rounds, s);
+    const int launched = wave == 0 ? split_scan<0>(e, dm, rounds, s) : split_scan<1>(e, dm, rounds, s);
     if (launched < 0) return fail("modisp_b200 CUDA: event record failed in the split scan");
     nl += launched;
   } else {
     e->sp_timed = 0;
     const dim3 grid(d.fp32 ? e->scan_blocks32 : e->scan_blocks64), block(32 * e->scan_warps);
     const size_t sm = d.fp32 ? e->scan_smem32 : e->scan_smem64;
-    if (d.fp32 && wave == 0) scan<float, 0><<<grid, block, sm, s>>>(d, d.trace_list, C_SCAN_CURSOR, C_NTRACE);
-    else if (d.fp32) scan<float, 1><<<grid, block, sm, s>>>(d, d.trace_list, C_SCAN_CURSOR, C_NTRACE);
-    else if (wave == 0) scan<double, 0><<<grid, block, sm, s>>>(d, d.trace_list, C_SCAN_CURSOR, C_NTRACE);
-    else scan<double, 1><<<grid, block, sm, s>>>(d, d.trace_list, C_SCAN_CURSOR, C_NTRACE);
+    if (d.fp32 && wave == 0) scan<float, 0><<<grid, block, sm, s>>>(dm, d.trace_list, C_SCAN_CURSOR, C_NTRACE);
+    else if (d.fp32) scan<float, 1><<<grid, block, sm, s>>>(dm, d.trace_list, C_SCAN_CURSOR, C_NTRACE);
+    else if (wave == 0) scan<double, 0><<<grid, block, sm, s>>>(dm, d.trace_list, C_SCAN_CURSOR, C_NTRACE);
+    else scan<double, 1><<<grid, block, sm, s>>>(dm, d.trace_list, C_SCAN_CURSOR, C_NTRACE);
     ++nl;
   }
   MD200_CK(cudaGetLastError());
   MD200_CK(mark(3));
+  if (dm.model_lists) {
+    list_brackets<<<model_blocks, 128, 0, s>>>(d);
+    ++nl;
+  }
   refine<<<e->list_blocks, 128, 0, s>>>(d);
   ++nl;
   MD200_CK(cudaGetLastError());
@@ -491,11 +504,15 @@ int enqueue(md200_engine *e, const double *h, const double *vp, const double *vs
     MD200_CK(mark(6));
   }
   MD200_CK(mark(7));
-  assemble<<<(nt + 255) / 256, 256, 0, s>>>(d);
+  assemble<<<(nt + 255) / 256, 256, 0, s>>>(dm);
   ++nl;
   MD200_CK(cudaGetLastError());
   MD200_CK(mark(8));
   if (d.group) {
+    if (dm.model_lists) {
+      list_roots<<<model_blocks, 128, 0, s>>>(d);
+      ++nl;
+    }
     group_velocity<<<e->list_blocks, 128, 0, s>>>(d);
     ++nl;
     MD200_CK(cudaGetLastError());

@@ -60,6 +60,7 @@ struct Dev {
   // geometry of this run
   int B, Lmax, Ls, T, nmodes, K, KB, wave, fp32, nlog, nkmax, nsmax;
   int n_traces, group;
+  int model_lists;  // this pass's brackets and roots are listed model by model (list_brackets, list_roots)
   long long jmax;   // scan points per trace before the workspace flag
   double tol, accept, close_rtol, density;
   // inputs (device)

@@ -351,7 +351,7 @@ __device__ __forceinline__ void split_publish(const Dev &d, int t, const ScanSta
   if (publish) {
     d.nbr[t] = st.nbr;
     if (st.tfl) atomicOr(&d.tflags[t], st.tfl);
-    if (!(st.tfl & TRACE_SEARCH_UNCONVERGED)) n = st.nbr;
+    if (!d.model_lists && !(st.tfl & TRACE_SEARCH_UNCONVERGED)) n = st.nbr;
   }
   const int base = warp_append(&d.ctr[C_NREFINE], n, lane);
   for (int k = 0; k < n; ++k) d.refine_list[base + k] = t * d.KB + k;
@@ -579,7 +579,7 @@ __global__ void __launch_bounds__(128) split_zoom(Dev d, int p) {
         d.sp_act[1 - p][atomicAdd(&d.ctr[C_SP_ACT0 + 1 - p], 1)] = t;
       }
     }
-    if (last || st.nbr >= x.K) {
+    if (!d.model_lists && (last || st.nbr >= x.K)) {
       int base = 0;
       if (lane == 0 && !(st.tfl & TRACE_SEARCH_UNCONVERGED)) base = atomicAdd(&d.ctr[C_NREFINE], st.nbr);
       base = __shfl_sync(FULL, base, 0);
