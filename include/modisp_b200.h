@@ -93,6 +93,12 @@ void md200_default_options(md200_options *options);
 md200_engine *md200_create(int device, int capacity, int layers, int periods, int nmodes,
                            const md200_options *options);
 
+/* The same engine without the pinned staging buffers of the host-array runs: for
+ * callers of the device-pointer and ragged runs (md200_run allocates them when it
+ * is called first). */
+md200_engine *md200_create_device(int device, int capacity, int layers, int periods, int nmodes,
+                                  const md200_options *options);
+
 /* Replaces QeSolver.run(...) (cpp/cuda/qe.cu:1060-1119) with host arrays: copies
  * inputs to the device, solves, copies outputs back and synchronises.
  *   thickness, vp, vs, rho : [models, layers]
@@ -317,6 +323,15 @@ typedef struct {
  * reliability.py:7-9 (log gap) and :107-144 (period walk). */
 int md200_reliability_plan(const double *periods, int T, double max_log_period_gap,
                            md200_period_plan *plan, int32_t *order);
+
+/* Masks of a result on host arrays (python/modisp/__init__.py:100-139): velocity
+ * [models][K][T] (float when `single`, else double), flags and counts [models][T].
+ * Outputs (0/1 bytes, status 0..3): mode_mask, close_mask and status [models][K][T],
+ * close_risk and approximate [models][T]; with `group`, group_mask [models][K][T]. */
+int md200_package(const void *velocity, int single, const uint32_t *flags, const int32_t *counts, int models, int K,
+                  int T, double close_rtol, uint8_t *mode_mask, uint8_t *close_mask, uint8_t *close_risk,
+                  uint8_t *approximate, uint8_t *status, const double *group, const uint32_t *group_flags,
+                  uint8_t *group_mask);
 
 /* The checks on host arrays: velocity [B][K][T] (positive or NaN), trace_flags
  * [B][T] (NULL: none), root_count [B][T] (NULL: finite roots per trace), plan and

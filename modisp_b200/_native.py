@@ -60,6 +60,8 @@ _I = ctypes.c_int
 EXPORTS = {
     "md200_default_options": (None, [ctypes.POINTER(Options)]),
     "md200_create": (_P, [_I, _I, _I, _I, _I, ctypes.POINTER(Options)]),
+    "md200_create_device": (_P, [_I, _I, _I, _I, _I, ctypes.POINTER(Options)]),
+    "md200_package": (_I, [_P, _I, _P, _P, _I, _I, _I, _D, _P, _P, _P, _P, _P, _P, _P, _P]),
     "md200_run": (_I, [_P, _P, _P, _P, _P, _I, _P, _P, _D, _D, _I, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _I]),
     "md200_run_device": (_I, [_P, _P, _P, _P, _P, _I, _P, _P, _D, _D, _I, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P,
                               _P]),
@@ -175,12 +177,12 @@ class Engine:
     """Owning handle of one md200_engine."""
 
     def __init__(self, device: int, capacity: int, layers: int, periods: int, nmodes: int,
-                 options: Options):
+                 options: Options, staging: bool = True):
         self.device, self.capacity, self.layers = int(device), int(capacity), int(layers)
         self.periods, self.nmodes = int(periods), int(nmodes)
         self.options = options
-        handle = lib().md200_create(self.device, self.capacity, self.layers, self.periods, self.nmodes,
-                                    ctypes.byref(options))
+        create = lib().md200_create if staging else lib().md200_create_device
+        handle = create(self.device, self.capacity, self.layers, self.periods, self.nmodes, ctypes.byref(options))
         if not handle:
             raise RuntimeError(last_error())
         self._handle = handle
@@ -410,6 +412,31 @@ def continuity_screen(periods, velocity, prediction=None, bilateral=True, device
     check(lib().md200_continuity_screen(int(device), ptr(p), T, ptr(v), B, K, ptr(pred), int(single),
                                         int(bool(bilateral)), ptr(flags), ctypes.byref(sus)))
     return flags, bool(sus.value)
+
+
+def package(velocity, flags, counts, close_rtol, group=None, group_flags=None):
+    """Masks of a result (md200_package): mode_mask, close_mask, status [B, K, T], close_risk and
+    approximate [B, T], group_mask [B, K, T] or None; None where the arrays are not the engine's
+    own types and layout."""
+    arrays = [(velocity, (np.float64, np.float32)), (flags, (np.uint32,)), (counts, (np.int32,))]
+    if group is not None:
+        arrays += [(group, (np.float64,)), (group_flags, (np.uint32,))]
+    for x, types in arrays:
+        if not isinstance(x, np.ndarray) or x.dtype not in types or not x.flags.c_contiguous:
+            return None
+    if velocity.ndim != 3 or not velocity.size or _lib is None:
+        return None
+    B, K, T = velocity.shape
+    if flags.shape != (B, T) or counts.shape != (B, T) or \
+            (group is not None and not group.shape == group_flags.shape == velocity.shape):
+        return None
+    cells = [np.empty(velocity.shape, bool) for _ in range(2 if group is None else 3)]
+    traces = [np.empty((B, T), bool) for _ in range(2)]
+    status = np.empty(velocity.shape, np.uint8)
+    check(lib().md200_package(ptr(velocity), int(velocity.dtype == np.float32), ptr(flags), ptr(counts), B, K, T,
+                              float(close_rtol), ptr(cells[0]), ptr(cells[1]), ptr(traces[0]), ptr(traces[1]),
+                              ptr(status), ptr(group), ptr(group_flags), ptr(cells[2]) if group is not None else None))
+    return cells[0], cells[1], status, traces[0], traces[1], cells[2] if group is not None else None
 
 
 def group_roots(h, vp, vs, rho, wave, period, roots, modes, close_rtol=.005):

@@ -83,6 +83,28 @@ class PredictionFlag(IntFlag):
     REVIEW = 4096
 
 
+def _masks(velocity, flags, counts, close_root_rtol, group_velocity, group_velocity_flags):
+    """The masks of a result in numpy, for arrays that are not the engine's own types and layout
+    (``_native.package`` makes the same ones in one pass over the cells)."""
+    approximate = (flags & (TRACE_APPROXIMATE_SEARCH | TRACE_CONTINUATION_APPROXIMATE)) != 0
+    close_root_mask = np.zeros(velocity.shape, dtype=bool)
+    if velocity.shape[1] > 1:
+        gaps = np.diff(velocity, axis=1)
+        close = np.isfinite(gaps) & (gaps <= close_root_rtol * velocity[:, 1:, :])
+        close_root_mask[:, :-1, :] |= close
+        close_root_mask[:, 1:, :] |= close
+    close_root_risk = ((flags & TRACE_CLOSE_ROOT_RISK) != 0) | np.any(close_root_mask, axis=1)
+    mode_mask = np.isfinite(velocity)
+    status = np.where(mode_mask, SolveStatus.VALID,
+                      np.where((flags[:, None, :] & (TRACE_SEARCH_UNCONVERGED | TRACE_UNRESOLVED_BRACKET)) != 0,
+                               SolveStatus.UNRESOLVED, SolveStatus.NOT_FOUND)).astype(np.uint8)
+    rejected = (np.isnan(velocity) & ((flags[:, None, :] & TRACE_F_REJECTED) != 0)
+                & (np.arange(velocity.shape[1])[None, :, None] < counts[:, None, :]))
+    status[rejected] = SolveStatus.REJECTED
+    group_mask = None if group_velocity is None else np.isfinite(group_velocity) & (group_velocity_flags == 0)
+    return mode_mask, close_root_mask, status, close_root_risk, approximate, group_mask
+
+
 class DispersionBatch:
     """Result of one solve (python/modisp/__init__.py:71-139): the same fields and masks."""
 
@@ -107,9 +129,6 @@ class DispersionBatch:
         self.close_root_rtol = float(close_root_rtol)
         self.group_velocity = group_velocity
         self.group_velocity_flags = group_velocity_flags
-        self.group_velocity_mask = (None if group_velocity is None
-                                    else np.isfinite(group_velocity) & (group_velocity_flags == 0))
-        self.group_velocity_valid = self.group_velocity_mask
         self.prediction_flags = prediction_flags
         self.continuity_flags = continuity_flags
         self.group_rtol = group_rtol
@@ -117,17 +136,13 @@ class DispersionBatch:
         self.frequency_strategy_used = frequency_strategy_used
         self.frequency_strategy_reason = frequency_strategy_reason
         self.anchor_stride = int(anchor_stride)
-        self.approximate_search = (flags & (TRACE_APPROXIMATE_SEARCH | TRACE_CONTINUATION_APPROXIMATE)) != 0
+        masks = _native.package(velocity, flags, counts, self.close_root_rtol, group_velocity, group_velocity_flags)
+        if masks is None:
+            masks = _masks(velocity, flags, counts, self.close_root_rtol, group_velocity, group_velocity_flags)
+        self.mode_mask, self.close_root_mask, self.status, self.close_root_risk, self.approximate_search, group = masks
+        self.group_velocity_mask = self.group_velocity_valid = group
         self.mode_index_uncertain = self.approximate_search.copy()
-        self.close_root_mask = np.zeros(velocity.shape, dtype=bool)
-        if nmodes > 1:
-            gaps = np.diff(velocity, axis=1)
-            close = np.isfinite(gaps) & (gaps <= self.close_root_rtol * velocity[:, 1:, :])
-            self.close_root_mask[:, :-1, :] |= close
-            self.close_root_mask[:, 1:, :] |= close
-        self.close_root_risk = ((flags & TRACE_CLOSE_ROOT_RISK) != 0) | np.any(self.close_root_mask, axis=1)
         self.potentially_ambiguous = self.mode_index_uncertain | self.close_root_risk
-        self.mode_mask = np.isfinite(velocity)
         self.trace_flags = flags
         self.numerical_flags = flags & np.uint32(0xFFFFFFFF ^ (TRACE_RANGE_TRUNCATED | TRACE_AUTO_RELAXED))
         self.search_level = levels
@@ -135,12 +150,6 @@ class DispersionBatch:
         self.search_bounds = np.array(bounds, copy=True)
         self.backend_used = backend
         self.backend_reason = reason
-        self.status = np.where(self.mode_mask, SolveStatus.VALID,
-                               np.where((flags[:, None, :] & (TRACE_SEARCH_UNCONVERGED | TRACE_UNRESOLVED_BRACKET)) != 0,
-                                        SolveStatus.UNRESOLVED, SolveStatus.NOT_FOUND)).astype(np.uint8)
-        rejected = (np.isnan(velocity) & ((flags[:, None, :] & TRACE_F_REJECTED) != 0)
-                    & (np.arange(nmodes)[None, :, None] < counts[:, None, :]))
-        self.status[rejected] = SolveStatus.REJECTED
         self.mode_convention = "ascending roots in the reported search interval"
 
     @property
@@ -345,11 +354,14 @@ class Solver:
             limit = max(1, int(0.4 * free) // per_model)
         return max(1, min(B, limit, self.chunk_size or B))
 
+    def _key(self, L, T, nmodes, continuation):
+        return (self.device, L, T, int(nmodes), self.accuracy, self.close_root_rtol, self.precision,
+                self.group_velocity, bool(continuation), self.anchor_stride, self.continuity_check,
+                tuple(sorted(self.tuning.items())))
+
     def _engine_for(self, capacity, L, T, nmodes, continuation=False):
         from . import plugin
-        key = (self.device, L, T, int(nmodes), self.accuracy, self.close_root_rtol, self.precision,
-               self.group_velocity, bool(continuation), self.anchor_stride, self.continuity_check,
-               tuple(sorted(self.tuning.items())))
+        key = self._key(L, T, nmodes, continuation)
         if self._engine is not None and self._engine_key[0] == key and self._engine_key[1] >= capacity:
             return self._engine, False
         self.close()
@@ -422,19 +434,25 @@ class Solver:
         bounds_in = np.zeros((B, 2))
         bounds_in[:, 0] = self.cmin if self.cmin is not None else 0.
         bounds_in[:, 1] = self.cmax if self.cmax is not None else np.inf
-        capacity = self._capacity(B, L, per.size, nmodes)
+        if self._engine is not None and self.workspace_bytes is None and self.chunk_size is None and \
+                self._engine_key == (self._key(L, per.size, nmodes, continuation), B):
+            capacity = B  # the engine of the last call fits: no look at the free memory
+        else:
+            capacity = self._capacity(B, L, per.size, nmodes)
         engine, allocated = self._engine_for(capacity, L, per.size, nmodes, continuation)
         dtype = np.float32 if self.precision == "float32" else np.float64
-        velocity = np.empty((B, nmodes, per.size), dtype=dtype)
-        flags = np.empty((B, per.size), np.uint32)
-        levels = np.empty((B, per.size), np.int32)
-        counts = np.empty((B, per.size), np.int32)
-        bounds = np.empty((B, 2))
-        group = np.empty((B, nmodes, per.size)) if self.group_velocity else None
-        gflags = np.empty((B, nmodes, per.size), np.uint32) if self.group_velocity else None
         # the continuity screen runs in the FP32-scan engine (continuity_check)
         screened = self.precision != "float64" and self.continuity_check
-        cflags = np.empty((B, per.size), np.uint8) if screened else None
+        group = gflags = cflags = None
+        if B > capacity:  # (one chunk: the engine's own output arrays)
+            velocity = np.empty((B, nmodes, per.size), dtype=dtype)
+            flags = np.empty((B, per.size), np.uint32)
+            levels = np.empty((B, per.size), np.int32)
+            counts = np.empty((B, per.size), np.int32)
+            bounds = np.empty((B, 2))
+            group = np.empty((B, nmodes, per.size)) if self.group_velocity else None
+            gflags = np.empty((B, nmodes, per.size), np.uint32) if self.group_velocity else None
+            cflags = np.empty((B, per.size), np.uint8) if screened else None
         # PredictionFlag words: BYPASSED (8) unless continuation assigns them
         pflags = (np.full((B, per.size), 8, np.uint32) if self.frequency_strategy == "anchor_continuation"
                   else None)
@@ -446,16 +464,25 @@ class Solver:
             out = engine._engine.run(h[start:end], a[start:end], b[start:end], r[start:end], per,
                                      bounds_in[start:end], self.c_tol_rel, self.f_accept, wave_code,
                                      group=self.group_velocity, continuity=screened, prediction=continuation)
-            velocity[start:end] = out["velocity"]
-            flags[start:end] = out["flags"]
-            levels[start:end] = out["levels"]
-            counts[start:end] = out["counts"]
-            bounds[start:end] = out["bounds"]
-            if self.group_velocity:
-                group[start:end] = out["group_velocity"]
-                gflags[start:end] = out["group_velocity_flags"]
-            if screened:
-                cflags[start:end] = out["continuity_flags"]
+            if B <= capacity:
+                velocity, flags, levels, counts, bounds = (out[k] for k in ("velocity", "flags", "levels", "counts",
+                                                                            "bounds"))
+                velocity = velocity.astype(dtype, copy=False)
+                if self.group_velocity:
+                    group, gflags = out["group_velocity"], out["group_velocity_flags"]
+                if screened:
+                    cflags = out["continuity_flags"]
+            else:
+                velocity[start:end] = out["velocity"]
+                flags[start:end] = out["flags"]
+                levels[start:end] = out["levels"]
+                counts[start:end] = out["counts"]
+                bounds[start:end] = out["bounds"]
+                if self.group_velocity:
+                    group[start:end] = out["group_velocity"]
+                    gflags[start:end] = out["group_velocity_flags"]
+                if screened:
+                    cflags[start:end] = out["continuity_flags"]
             if continuation:
                 pflags[start:end] = out["prediction_flags"]
             for k, v in out["stats"].items():

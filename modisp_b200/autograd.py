@@ -63,7 +63,8 @@ class DifferentiableSolver:
         o = _native.default_options()
         o.single_precision = 1 if precision == "mixed" else 0
         o.group_velocity = 1
-        self.engine = _native.Engine(self.device, self.capacity, self.layers, per.size, self.nmodes, o)
+        self.engine = _native.Engine(self.device, self.capacity, self.layers, per.size, self.nmodes, o,
+                                     staging=False)
 
     def _inputs(self, thickness, vp, vs, rho):
         B = thickness.shape[0] if thickness.dim() == 2 else -1

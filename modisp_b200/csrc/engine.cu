@@ -130,6 +130,13 @@ struct md200_engine {
   long long *rg_outbase = nullptr;
   double *rg_periods = nullptr;
   std::vector<void *> owned;
+  // workspace arrays of setup(), laid out in one allocation (plan_alloc, commit_plan)
+  struct Planned {
+    void **p;
+    size_t offset;
+  };
+  std::vector<Planned> plan;
+  size_t plan_bytes = 0;
   // host-path pipelining: chunks of models solved on `stream`, each chunk's outputs
   // copied back on `copy_stream` once its solve has ended (solved_ev) while the next
   // chunk is solved; chunk_ev marks the end of a chunk's copies
@@ -158,6 +165,34 @@ template <class T>
 int own_alloc(md200_engine *e, T **p, size_t count) {
   MD200_CK(dalloc(p, count));
   e->owned.push_back(*p);
+  return 0;
+}
+
+// setup()'s arrays come from one allocation: some fifty allocations and frees per
+// engine cost a call that makes its own engine (a ragged batch) more than its
+// solve.  1,000 models of 30-100 layers: 87 -> 34 ms a call, without the staging
+// below as well.
+template <class T>
+int plan_alloc(md200_engine *e, T **p, size_t count) {
+  *p = nullptr;
+  e->plan.push_back({reinterpret_cast<void **>(p), e->plan_bytes});
+  e->plan_bytes += (std::max<size_t>(count, 1) * sizeof(T) + 255) & ~size_t(255);
+  return 0;
+}
+int commit_plan(md200_engine *e) {
+  unsigned char *base = nullptr;
+  if (own_alloc(e, &base, e->plan_bytes)) return 1;
+  for (const auto &x : e->plan) *x.p = base + x.offset;
+  e->plan.clear();
+  return 0;
+}
+
+// Pinned staging of the host-array runs, allocated with the engine or by the
+// first of them (engines that only take device pointers or ragged batches have
+// no use for it).
+int need_staging(md200_engine *e) {
+  if (e->pinned) return 0;
+  MD200_CK(cudaMallocHost(reinterpret_cast<void **>(&e->pinned), e->pinned_bytes));
   return 0;
 }
 
@@ -191,7 +226,7 @@ size_t scan_smem(int warps, int Ls, size_t elem) {
   return static_cast<size_t>(warps) * (tab + 32 * sizeof(double));
 }
 
-int setup(md200_engine *e) {
+int setup(md200_engine *e, bool staging) {
   MD200_CK(cudaSetDevice(e->device));
   MD200_CK(cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking));
   MD200_CK(cudaStreamCreateWithFlags(&e->copy_stream, cudaStreamNonBlocking));
@@ -212,60 +247,61 @@ int setup(md200_engine *e) {
   d.fp32 = e->o.single_precision ? 1 : 0;
   d.group = e->o.group_velocity ? 1 : 0;
   const size_t nt = static_cast<size_t>(B) * T;
-  if (own_alloc(e, &d.mL, B) || own_alloc(e, &d.mwater, B) || own_alloc(e, &d.mstate, B) ||
-      own_alloc(e, &d.mlo, B) || own_alloc(e, &d.mhi, B) || own_alloc(e, &d.malpha, B) ||
-      own_alloc(e, &d.mstart, B) ||
-      own_alloc(e, &d.mtail, 2 * static_cast<size_t>(B)) || own_alloc(e, &d.tail, 2 * nt) ||
-      own_alloc(e, &d.layer64, static_cast<size_t>(B) * ROWS * d.Ls) ||
-      own_alloc(e, &d.layer32, static_cast<size_t>(B) * ROWS * d.Ls) ||
-      own_alloc(e, &d.knot, static_cast<size_t>(B) * d.nkmax) || own_alloc(e, &d.nknot, B) ||
-      own_alloc(e, &d.seed, static_cast<size_t>(B) * d.nsmax) || own_alloc(e, &d.nseed, B) ||
-      own_alloc(e, &d.nbr, nt) || own_alloc(e, &d.tflags, nt) ||
-      own_alloc(e, &d.tr_model, nt) || own_alloc(e, &d.tr_stride, nt) || own_alloc(e, &d.tr_modes, nt) ||
-      own_alloc(e, &d.tr_period, nt) || own_alloc(e, &d.tr_out, nt) ||
-      own_alloc(e, &d.slot, nt * d.KB * SLOT) ||
-      own_alloc(e, &d.trace_list, nt) || own_alloc(e, &d.repair_list, nt) ||
-      own_alloc(e, &d.refine_list, 2 * nt * d.KB) ||
-      own_alloc(e, &d.group_list, nt * nm) || own_alloc(e, &d.ctr, C_COUNT) ||
-      own_alloc(e, &e->d_stats, static_cast<size_t>(MD200_STAT_COUNT) * md200_engine::MAX_CHUNKS))
+  if (plan_alloc(e, &d.mL, B) || plan_alloc(e, &d.mwater, B) || plan_alloc(e, &d.mstate, B) ||
+      plan_alloc(e, &d.mlo, B) || plan_alloc(e, &d.mhi, B) || plan_alloc(e, &d.malpha, B) ||
+      plan_alloc(e, &d.mstart, B) ||
+      plan_alloc(e, &d.mtail, 2 * static_cast<size_t>(B)) || plan_alloc(e, &d.tail, 2 * nt) ||
+      plan_alloc(e, &d.layer64, static_cast<size_t>(B) * ROWS * d.Ls) ||
+      plan_alloc(e, &d.layer32, static_cast<size_t>(B) * ROWS * d.Ls) ||
+      plan_alloc(e, &d.knot, static_cast<size_t>(B) * d.nkmax) || plan_alloc(e, &d.nknot, B) ||
+      plan_alloc(e, &d.seed, static_cast<size_t>(B) * d.nsmax) || plan_alloc(e, &d.nseed, B) ||
+      plan_alloc(e, &d.nbr, nt) || plan_alloc(e, &d.tflags, nt) ||
+      plan_alloc(e, &d.tr_model, nt) || plan_alloc(e, &d.tr_stride, nt) || plan_alloc(e, &d.tr_modes, nt) ||
+      plan_alloc(e, &d.tr_period, nt) || plan_alloc(e, &d.tr_out, nt) ||
+      plan_alloc(e, &d.slot, nt * d.KB * SLOT) ||
+      plan_alloc(e, &d.trace_list, nt) || plan_alloc(e, &d.repair_list, nt) ||
+      plan_alloc(e, &d.refine_list, 2 * nt * d.KB) ||
+      plan_alloc(e, &d.group_list, nt * nm) || plan_alloc(e, &d.ctr, C_COUNT) ||
+      plan_alloc(e, &e->d_stats, static_cast<size_t>(MD200_STAT_COUNT) * md200_engine::MAX_CHUNKS))
     return 1;
   // host-path device buffers
-  if (own_alloc(e, &e->in_h, static_cast<size_t>(B) * L) ||
-      own_alloc(e, &e->in_vp, static_cast<size_t>(B) * L) ||
-      own_alloc(e, &e->in_vs, static_cast<size_t>(B) * L) ||
-      own_alloc(e, &e->in_rho, static_cast<size_t>(B) * L) || own_alloc(e, &e->in_per, T) ||
-      own_alloc(e, &e->in_bounds, static_cast<size_t>(B) * 2) ||
-      own_alloc(e, &e->out_vel, nt * nm) || own_alloc(e, &e->out_grp, nt * nm) ||
-      own_alloc(e, &e->out_gflags, nt * nm) || own_alloc(e, &e->out_flags, nt) ||
-      own_alloc(e, &e->out_pred, nt) || own_alloc(e, &e->out_levels, nt) ||
-      own_alloc(e, &e->out_counts, nt) || own_alloc(e, &e->out_cflags, nt))
+  if (plan_alloc(e, &e->in_h, static_cast<size_t>(B) * L) ||
+      plan_alloc(e, &e->in_vp, static_cast<size_t>(B) * L) ||
+      plan_alloc(e, &e->in_vs, static_cast<size_t>(B) * L) ||
+      plan_alloc(e, &e->in_rho, static_cast<size_t>(B) * L) || plan_alloc(e, &e->in_per, T) ||
+      plan_alloc(e, &e->in_bounds, static_cast<size_t>(B) * 2) ||
+      plan_alloc(e, &e->out_vel, nt * nm) || plan_alloc(e, &e->out_grp, nt * nm) ||
+      plan_alloc(e, &e->out_gflags, nt * nm) || plan_alloc(e, &e->out_flags, nt) ||
+      plan_alloc(e, &e->out_pred, nt) || plan_alloc(e, &e->out_levels, nt) ||
+      plan_alloc(e, &e->out_counts, nt) || plan_alloc(e, &e->out_cflags, nt))
     return 1;
   // roots and counts of continuity suspects before their FP64 re-scan
   if (d.fp32 && e->o.continuity_check &&
-      (own_alloc(e, &d.cold, nt * nm) || own_alloc(e, &d.ccount, nt)))
+      (plan_alloc(e, &d.cold, nt * nm) || plan_alloc(e, &d.ccount, nt)))
     return 1;
   // split FP32 scan: active lists, per-trace state, per-sample buffers
   if (d.fp32) {
     d.sp_cap = static_cast<int>(std::min<size_t>(nt, SPLIT_ACTIVE_MAX));
     const size_t ns = static_cast<size_t>(d.sp_cap) * SPLIT_SAMPLES;
-    if (own_alloc(e, &d.sp_act[0], d.sp_cap) || own_alloc(e, &d.sp_act[1], d.sp_cap) ||
-        own_alloc(e, &d.sp_state, nt) || own_alloc(e, &d.sp_s, ns) || own_alloc(e, &d.sp_tr, d.sp_cap) ||
-        own_alloc(e, &d.sp_kf, nt) ||
-        own_alloc(e, &d.sp_redo, ns) || own_alloc(e, &d.sp_zoom, d.sp_cap) ||
-        own_alloc(e, &d.sp_zarg, static_cast<size_t>(d.sp_cap) * 8))
+    if (plan_alloc(e, &d.sp_act[0], d.sp_cap) || plan_alloc(e, &d.sp_act[1], d.sp_cap) ||
+        plan_alloc(e, &d.sp_state, nt) || plan_alloc(e, &d.sp_s, ns) || plan_alloc(e, &d.sp_tr, d.sp_cap) ||
+        plan_alloc(e, &d.sp_kf, nt) ||
+        plan_alloc(e, &d.sp_redo, ns) || plan_alloc(e, &d.sp_zoom, d.sp_cap) ||
+        plan_alloc(e, &d.sp_zarg, static_cast<size_t>(d.sp_cap) * 8))
       return 1;
   }
   // anchor continuation: plan, anchor slopes and safety, target and root lists
   if (e->o.continuation &&
-      (own_alloc(e, &d.crole, nt) || own_alloc(e, &d.cleft, nt) || own_alloc(e, &d.cright, nt) ||
-       own_alloc(e, &d.cslope, nt * d.KB) || own_alloc(e, &d.csafe, nt) || own_alloc(e, &d.cont_list, nt) ||
-       own_alloc(e, &d.croot_list, nt * d.KB) || own_alloc(e, &d.ccode, nt * d.KB)))
+      (plan_alloc(e, &d.crole, nt) || plan_alloc(e, &d.cleft, nt) || plan_alloc(e, &d.cright, nt) ||
+       plan_alloc(e, &d.cslope, nt * d.KB) || plan_alloc(e, &d.csafe, nt) || plan_alloc(e, &d.cont_list, nt) ||
+       plan_alloc(e, &d.croot_list, nt * d.KB) || plan_alloc(e, &d.ccode, nt * d.KB)))
     return 1;
   e->pinned_bytes = sizeof(double) * (4 * static_cast<size_t>(B) * L + T + 2 * static_cast<size_t>(B)) +
                     nt * nm * (2 * sizeof(double) + sizeof(unsigned)) + nt * 4 * sizeof(int) + nt +
                     md200_engine::MAX_CHUNKS * MD200_STAT_COUNT * sizeof(unsigned long long) +
                     2 * sizeof(double) * B + 64;
-  MD200_CK(cudaMallocHost(reinterpret_cast<void **>(&e->pinned), e->pinned_bytes));
+  if (commit_plan(e)) return 1;
+  if (staging && need_staging(e)) return 1;
 
   // launch shapes
   int sms = 148;
@@ -703,6 +739,57 @@ __global__ void fma_chains(T *out, int iters, T a, T b) {
   if (sum == static_cast<T>(-1.2345)) out[0] = sum;  // keeps the chains live
 }
 
+// ---------------------------------------------------------------------------
+// Result masks of a batch (python/modisp/__init__.py:100-139): one pass over the
+// cells on up to 8 host threads, with numpy's arithmetic of the array's own type.
+// ---------------------------------------------------------------------------
+struct PackageArgs {
+  const uint32_t *flags;
+  const int32_t *counts;
+  int K, T;
+  double close_rtol;
+  uint8_t *mode_mask, *close_mask, *close_risk, *approximate, *status;
+  const double *group;
+  const uint32_t *group_flags;
+  uint8_t *group_mask;
+};
+template <class V>
+void package_models(const V *velocity, const PackageArgs &a, size_t b0, size_t b1) {
+  const size_t K = a.K, T = a.T;
+  const V rtol = static_cast<V>(a.close_rtol);
+  for (size_t b = b0; b < b1; ++b) {
+    const uint32_t *fl = a.flags + b * T;
+    uint8_t *risk = a.close_risk + b * T;
+    for (size_t f = 0; f < T; ++f) {
+      risk[f] = (fl[f] & 4096u) != 0;                                  // TRACE_CLOSE_ROOT_RISK
+      a.approximate[b * T + f] = (fl[f] & (2048u | 65536u)) != 0;      // ..._APPROXIMATE(_SEARCH)
+    }
+    for (size_t k = 0; k < K; ++k) {
+      const size_t o = (b * K + k) * T;
+      const V *v = velocity + o;
+      for (size_t f = 0; f < T; ++f) {
+        const bool finite = std::isfinite(v[f]);
+        const bool rejected = std::isnan(v[f]) && (fl[f] & 128u) && static_cast<int32_t>(k) < a.counts[b * T + f];
+        a.mode_mask[o + f] = finite;
+        a.status[o + f] = rejected ? 3 : finite ? 0 : (fl[f] & 5u) ? 2 : 1;
+        bool close = false;
+        if (k > 0) {
+          const V gap = v[f] - v[f - T];
+          close = std::isfinite(gap) && gap <= rtol * v[f];
+        }
+        if (k + 1 < K) {
+          const V next = v[f + T], gap = next - v[f];
+          close = close || (std::isfinite(gap) && gap <= rtol * next);
+        }
+        a.close_mask[o + f] = close;
+        risk[f] |= close;
+      }
+      if (a.group)
+        for (size_t f = 0; f < T; ++f)
+          a.group_mask[o + f] = std::isfinite(a.group[o + f]) && a.group_flags[o + f] == 0;
+    }
+  }
+}
 }  // namespace
 
 extern "C" {
@@ -721,33 +808,54 @@ void md200_default_options(md200_options *o) {
   o->continuity_check = 1;
 }
 
+static md200_engine *create(int device, int capacity, int layers, int periods, int nmodes,
+                            const md200_options *options, bool staging) {
+  try {
+    if (capacity < 1 || layers < 1 || layers > 256 || periods < 1 || nmodes < 1 || nmodes > 256) {
+      fail("modisp_b200: invalid engine geometry (capacity >= 1, 1 <= layers <= 256, periods >= 1, "
+           "1 <= nmodes <= 256)");
+      return nullptr;
+    }
+    md200_engine *e = new (std::nothrow) md200_engine();
+    if (!e) {
+      fail("modisp_b200: out of host memory");
+      return nullptr;
+    }
+    e->device = device;
+    e->cap = capacity;
+    e->L = layers;
+    e->T = periods;
+    e->nmodes = nmodes;
+    if (options) e->o = *options;
+    else md200_default_options(&e->o);
+    bool failed = true;
+    try {
+      failed = setup(e, staging) != 0;
+    } catch (...) {
+      fail_exception();
+    }
+    if (failed) {
+      const std::string msg = g_error;
+      release(e);
+      delete e;
+      g_error = msg;
+      return nullptr;
+    }
+    return e;
+  } catch (...) {
+    fail_exception();
+    return nullptr;
+  }
+}
+
 md200_engine *md200_create(int device, int capacity, int layers, int periods, int nmodes,
                            const md200_options *options) {
-  if (capacity < 1 || layers < 1 || layers > 256 || periods < 1 || nmodes < 1 || nmodes > 256) {
-    fail("modisp_b200: invalid engine geometry (capacity >= 1, 1 <= layers <= 256, periods >= 1, "
-         "1 <= nmodes <= 256)");
-    return nullptr;
-  }
-  md200_engine *e = new (std::nothrow) md200_engine();
-  if (!e) {
-    fail("modisp_b200: out of host memory");
-    return nullptr;
-  }
-  e->device = device;
-  e->cap = capacity;
-  e->L = layers;
-  e->T = periods;
-  e->nmodes = nmodes;
-  if (options) e->o = *options;
-  else md200_default_options(&e->o);
-  if (setup(e)) {
-    const std::string msg = g_error;
-    release(e);
-    delete e;
-    g_error = msg;
-    return nullptr;
-  }
-  return e;
+  return create(device, capacity, layers, periods, nmodes, options, true);
+}
+
+md200_engine *md200_create_device(int device, int capacity, int layers, int periods, int nmodes,
+                                  const md200_options *options) {
+  return create(device, capacity, layers, periods, nmodes, options, false);
 }
 
 int md200_run_device(md200_engine *e, const double *h, const double *vp, const double *vs,
@@ -776,6 +884,7 @@ int md200_run(md200_engine *e, const double *h, const double *vp, const double *
     if (e->d.group && (!group || !group_flags))
       return fail("modisp_b200: group-velocity engine needs group output arrays");
     MD200_CK(cudaSetDevice(e->device));
+    if (need_staging(e)) return 1;
     // copies left in flight by a call that failed part-way write the staging buffer
     MD200_CK(cudaStreamSynchronize(e->copy_stream));
     const size_t B = models, L = e->L, T = e->T, nm = e->nmodes, nt = B * T;
@@ -1176,9 +1285,10 @@ int md200_device_count(void) {
 int md200_available(int device) {
   const int n = md200_device_count();
   if (device < 0 || device >= n) return 0;
-  cudaDeviceProp prop;
-  if (cudaGetDeviceProperties(&prop, device) != cudaSuccess) return 0;
-  return prop.major == 10 ? 1 : 0;
+  // (one attribute: the full property query takes 3 ms, most of a one-model call)
+  int major = 0;
+  if (cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device) != cudaSuccess) return 0;
+  return major == 10 ? 1 : 0;
 }
 
 int md200_set_device(int device) {
@@ -1291,6 +1401,36 @@ int md200_group_roots(const double *h, const double *vp, const double *vs, const
   } catch (...) {
     return fail_exception();
   }
+}
+
+// The masks of a packed result (package_models).
+int md200_package(const void *velocity, int single, const uint32_t *flags, const int32_t *counts, int models, int K,
+                  int T, double close_rtol, uint8_t *mode_mask, uint8_t *close_mask, uint8_t *close_risk,
+                  uint8_t *approximate, uint8_t *status, const double *group, const uint32_t *group_flags,
+                  uint8_t *group_mask) {
+  if (!velocity || !flags || !counts || models < 0 || K < 1 || T < 1 || !mode_mask || !close_mask || !close_risk ||
+      !approximate || !status || (group && (!group_flags || !group_mask)))
+    return fail("modisp_b200: missing input or output array");
+  const PackageArgs a{flags, counts, K, T, close_rtol, mode_mask, close_mask, close_risk, approximate, status,
+                      group, group_flags, group_mask};
+  const size_t B = models, cells = B * K * T;
+  auto part = [&](size_t b0, size_t b1) {
+    if (single) package_models(static_cast<const float *>(velocity), a, b0, b1);
+    else package_models(static_cast<const double *>(velocity), a, b0, b1);
+  };
+  const unsigned hw = std::thread::hardware_concurrency();
+  const size_t nth = std::max<size_t>(1, std::min<size_t>(std::min(8u, hw ? hw : 1u), cells >> 17));
+  std::vector<std::thread> pool;
+  size_t started = 1;
+  try {  // ranges without a thread are done here
+    pool.reserve(nth - 1);
+    for (; started < nth; ++started) pool.emplace_back(part, B * started / nth, B * (started + 1) / nth);
+  } catch (...) {
+  }
+  part(0, B / nth);
+  for (size_t t = started; t < nth; ++t) part(B * t / nth, B * (t + 1) / nth);
+  for (std::thread &th : pool) th.join();
+  return 0;
 }
 
 // ---------------------------------------------------------------------------

@@ -147,7 +147,7 @@ def dispersion_ragged(thickness, vp, vs, rho, periods, nmodes=5, wave="rayleigh"
     o.continuation = int(frequency_strategy == "anchor_continuation")
     o.anchor_stride = int(anchor_stride)
     cap = int(min(B, chunk_models))
-    engine = _native.Engine(device, cap, L, T_max, nm_max, o)
+    engine = _native.Engine(device, cap, L, T_max, nm_max, o, staging=False)
     try:
         for s in range(0, B, cap):
             e = min(B, s + cap)
