@@ -279,6 +279,7 @@ int setup(md200_engine *e, bool staging) {
   if (d.fp32 && e->o.continuity_check &&
       (plan_alloc(e, &d.cold, nt * nm) || plan_alloc(e, &d.ccount, nt)))
     return 1;
+  if (d.fp32 && plan_alloc(e, &d.pair32, static_cast<size_t>(B) * d.Ls * PAIR_ROW * 2)) return 1;
   // split FP32 scan: active lists, per-trace state, per-sample buffers
   if (d.fp32) {
     d.sp_cap = static_cast<int>(std::min<size_t>(nt, SPLIT_ACTIVE_MAX));
@@ -315,6 +316,8 @@ int setup(md200_engine *e, bool staging) {
   for (auto fn : {scan<float, 0>, scan<float, 1>})
     MD200_CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   static_cast<int>(std::max<size_t>(e->scan_smem32, 1024))));
+  MD200_CK(cudaFuncSetAttribute(split_eval32_pair, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                static_cast<int>(split_pair_smem(d.Ls, split_pair_buffers(d.Ls)))));
   int occ64 = 0, occ32 = 0;
   MD200_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ64, scan<double, 0>, 32 * e->scan_warps,
                                                          e->scan_smem64));
@@ -388,7 +391,7 @@ int split_scan(md200_engine *e, const Dev &d, int rounds, cudaStream_t s) {
   const int cap = d.sp_cap;
   const int fill_blocks = std::max(1, std::min((cap + 255) / 256, sms * 8));
   const int pos_blocks = std::max(1, std::min((cap + 3) / 4, sms * 16));
-  const int eval_blocks = sms * 16;
+  const int eval_blocks = sms * 16, buffers = split_pair_buffers(d.Ls);
   const int book_blocks = std::max(1, std::min((cap + 127) / 128, sms * 8));
   int nl = 0;
   for (int r = 0; r < rounds; ++r) {
@@ -399,7 +402,7 @@ int split_scan(md200_engine *e, const Dev &d, int rounds, cudaStream_t s) {
     if (!e->capturing && cudaEventRecord(e->sp_ev[2 * r], s) != cudaSuccess) return -1;
 #if MD200_SPLIT_PAIR
     if (WAVE == 0)
-      split_eval32_pair<<<sms * MD200_SPLIT_PAIR_GRID, 128, 0, s>>>(d, p);
+      split_eval32_pair<<<sms * MD200_SPLIT_PAIR_GRID, 128, split_pair_smem(d.Ls, buffers), s>>>(d, p, buffers);
     else
 #endif
       split_eval32<WAVE><<<eval_blocks, 128, 0, s>>>(d, p);

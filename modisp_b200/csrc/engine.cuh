@@ -74,6 +74,7 @@ struct Dev {
   double4 *tail;    // [n_traces][2]: FP64 (c, F, g, log-magnitude) at those positions
   double *layer64;  // [B][ROWS][Ls]
   float *layer32;   // [B][ROWS][Ls]
+  float *pair32;    // [B][Ls][PAIR_ROW][2]: the paired FP32 evaluation's layer records (FP32-scan engines)
   double4 *knot;    // [B][nkmax]: c, N(c), ln c, kink part of N over [c_i, c_i+1]
   int *nknot;
   double *seed;     // [B][nsmax]

@@ -265,6 +265,16 @@ __global__ void prep_models(Dev d, int sortcap, int automatic) {
         t64[q * Ls + r] = vals[q];
         t32[q * Ls + r] = static_cast<float>(vals[q]);
       }
+      if (d.fp32 && !d.wave) {  // the paired evaluation's record of this layer
+        const float h = static_cast<float>(vals[0]), vs2 = static_cast<float>(vals[3]), rho = static_cast<float>(vals[4]);
+        const float irho = static_cast<float>(vals[5]), nrho2 = -x_mul(rho, rho), nirho2 = -x_mul(irho, irho);
+        const float rec[PAIR_ROW] = {h,    static_cast<float>(vals[1]), static_cast<float>(vals[2]),
+                                     2.f * vs2, -2.f * vs2, rho, -rho, irho, -irho, nrho2, nirho2, 0.f};
+        float4 *out = reinterpret_cast<float4 *>(d.pair32 + (static_cast<size_t>(b) * Ls + r) * PAIR_ROW * 2);
+#pragma unroll
+        for (int q = 0; q < PAIR_ROW / 2; ++q)
+          out[q] = make_float4(rec[2 * q], rec[2 * q], rec[2 * q + 1], rec[2 * q + 1]);
+      }
     }
     L += __popc(mask);
   }

@@ -769,6 +769,12 @@ __device__ __forceinline__ float x_fma(float a, float b, float c) {
   return r;
 }
 
+__device__ __forceinline__ float x_ex2(float a) {
+  float r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
+  return r;
+}
+
 struct R1 {
   using V = float;
   static constexpr int NL = 1;
@@ -779,12 +785,11 @@ struct R1 {
   static __device__ __forceinline__ V splat(float a) { return a; }
   static __device__ __forceinline__ V neg(V a) { return -a; }
   static __device__ __forceinline__ V abs(V a) { return fabsf(a); }
-  static __device__ __forceinline__ M lt(V a, float b) { return a < b; }
+  static __device__ __forceinline__ M ltv(V a, V b) { return a < b; }
   static __device__ __forceinline__ M gt0(V a) { return a > 0.f; }
   static __device__ __forceinline__ V sel(M m, V a, V b) { return m ? a : b; }
   static __device__ __forceinline__ V rsqrt0(V a) { return a > 0.f ? rsqrtf(a) : 0.f; }
-  static __device__ __forceinline__ V expneg(V a) { return __expf(-a); }
-  static __device__ __forceinline__ V rint(V a) { return rintf(a); }
+  static __device__ __forceinline__ V ex2(V a) { return x_ex2(a); }
   static __device__ __forceinline__ void sincos(V r, V *s, V *c) { __sincosf(r, s, c); }
 };
 
@@ -822,12 +827,11 @@ struct R2 {
   static __device__ __forceinline__ V splat(float a) { return make_float2(a, a); }
   static __device__ __forceinline__ V neg(V a) { return make_float2(-a.x, -a.y); }
   static __device__ __forceinline__ V abs(V a) { return make_float2(fabsf(a.x), fabsf(a.y)); }
-  static __device__ __forceinline__ M lt(V a, float b) { return {a.x < b, a.y < b}; }
+  static __device__ __forceinline__ M ltv(V a, V b) { return {a.x < b.x, a.y < b.y}; }
   static __device__ __forceinline__ M gt0(V a) { return {a.x > 0.f, a.y > 0.f}; }
   static __device__ __forceinline__ V sel(M m, V a, V b) { return make_float2(m.x ? a.x : b.x, m.y ? a.y : b.y); }
   static __device__ __forceinline__ V rsqrt0(V a) { return make_float2(R1::rsqrt0(a.x), R1::rsqrt0(a.y)); }
-  static __device__ __forceinline__ V expneg(V a) { return make_float2(__expf(-a.x), __expf(-a.y)); }
-  static __device__ __forceinline__ V rint(V a) { return make_float2(rintf(a.x), rintf(a.y)); }
+  static __device__ __forceinline__ V ex2(V a) { return make_float2(x_ex2(a.x), x_ex2(a.y)); }
   static __device__ __forceinline__ void sincos(V r, V *s, V *c) {
     __sincosf(r.x, &s->x, &c->x);
     __sincosf(r.y, &s->y, &c->y);
@@ -838,9 +842,12 @@ struct R2 {
 // (exact for the |x| < 2^12 rad phases of the recurrences), then the
 // special-function unit (absolute error ~4e-7, far below the scan's
 // sign-decision threshold).
+// The nearest integer comes from adding and taking away 1.5 2^23 (exact below
+// 2^22): the conversion unit's rounding shares its port with the special functions.
 template <class P>
 __device__ __forceinline__ void sincos32(typename P::V x, typename P::V *s, typename P::V *c) {
-  const typename P::V n = P::rint(P::mul(x, P::splat(0.15915494309189535f)));
+  const typename P::V n =
+      P::add(P::add(P::mul(x, P::splat(0.15915494309189535f)), P::splat(12582912.f)), P::splat(-12582912.f));
   const typename P::V r = P::fma(n, P::splat(-1.7484555e-07f), P::fma(n, P::splat(-6.28318548f), x));
   P::sincos(r, s, c);
 }
@@ -861,65 +868,79 @@ __device__ __forceinline__ void apply32(typename P::V e[5], typename P::V k2, ty
   e[4] = P::fma(A, e4, P::fma(D, e3, P::fma(I, e2t, P::fma(C, e1, P::mul(Lm, e0)))));
 }
 
-// One standard Dunkin layer step (both waves trigonometric or scaled
-// hyperbolic, selected per lane), the algebra of rayleigh_layer_f32.  ka, kb,
-// gammk and the density powers are the layer's per-trace constants.  Returns
-// the exponent P + Q factored out of the evanescent waves.
+// A layer's constants on a lane type (both halves of a pair alike); nX is -X.
 template <class P>
-__device__ __forceinline__ typename P::V step32(typename P::V e[5], typename P::V k, typename P::V k2, float ka,
-                                                float kb, float gammk, float h, float rho, float irho, float rho2,
-                                                float irho2) {
+struct Layer32 {
   using V = typename P::V;
-  const V one = P::splat(1.f), zero = P::splat(0.f), half = P::splat(.5f), mhalf = P::splat(-.5f);
-  const V gam = P::mul(P::splat(gammk), k2);
-  const V Xa = P::mul(P::add(k, P::splat(ka)), P::abs(P::add(k, P::splat(-ka))));
-  const V Xb = P::mul(P::add(k, P::splat(kb)), P::abs(P::add(k, P::splat(-kb))));
-  const V ira = P::rsqrt0(Xa), irb = P::rsqrt0(Xb);
-  const V ra = P::mul(Xa, ira), rb = P::mul(Xb, irb);
-  const V p = P::mul(ra, P::splat(h)), q = P::mul(rb, P::splat(h));
-  V sp, cp, sq, cq;
-  sincos32<P>(p, &sp, &cp);
-  sincos32<P>(q, &sq, &cq);
-  const V ep = P::expneg(p), eq = P::expneg(q);
-  const V fp = P::mul(ep, ep), fq = P::mul(eq, eq);
-  const typename P::M pp = P::lt(k, ka), pq = P::lt(k, kb);  // propagating P / S
-  const V cosp = P::sel(pp, cp, P::fma(fp, half, half)), sinp = P::sel(pp, sp, P::fma(fp, mhalf, half));
-  const V cosq = P::sel(pq, cq, P::fma(fq, half, half)), sinq = P::sel(pq, sq, P::fma(fq, mhalf, half));
-  // sin(r h)/r -> h as r -> 0
-  const V wv = P::sel(P::gt0(Xa), P::mul(sinp, ira), P::splat(h));
-  const V yv = P::sel(P::gt0(Xb), P::mul(sinq, irb), P::splat(h));
-  const V tp = P::mul(ra, sinp), tq = P::mul(rb, sinq);
-  const V xv = P::sel(pp, P::neg(tp), tp), zv = P::sel(pq, P::neg(tq), tq);
-  const V a0 = P::mul(P::sel(pp, one, ep), P::sel(pq, one, eq));
-  const V expo = P::add(P::sel(pp, zero, p), P::sel(pq, zero, q));
-  const V cpcq = P::mul(cosp, cosq), cpy = P::mul(cosp, yv), cpz = P::mul(cosp, zv);
-  const V cqw = P::mul(cosq, wv), cqx = P::mul(cosq, xv);
-  const V xy = P::mul(xv, yv), xz = P::mul(xv, zv), wy = P::mul(wv, yv), wz = P::mul(wv, zv);
-  const V gmk = P::splat(gammk);
-  const V gm1 = P::add(gam, P::splat(-1.f)), twgm1 = P::add(gam, gm1);
-  const V gmgmk = P::mul(gam, gmk), gmgm1 = P::mul(gam, gm1), gm1sq = P::mul(gm1, gm1);
-  const V a0pq = P::add(a0, P::neg(cpcq));
-  const V k2gm1 = P::mul(k2, gm1), k2gm1sq = P::mul(k2, gm1sq);
-  V A = P::fma(P::mul(gmgm1, P::splat(-2.f)), a0pq, cpcq);
-  A = P::fma(P::neg(gmgmk), xz, A);
-  A = P::fma(P::neg(k2gm1sq), wy, A);
-  const V D = P::mul(P::fma(k2, cpy, P::neg(cqx)), P::splat(irho));
-  const V I = P::mul(P::fma(k2gm1, wy, P::fma(twgm1, a0pq, P::mul(gmk, xz))), P::splat(-irho));
-  const V C = P::mul(P::fma(P::neg(k2), cqw, cpz), P::splat(irho));
-  const V Lm = P::mul(P::fma(P::mul(k2, k2), wy, P::fma(P::mul(k2, P::splat(2.f)), a0pq, xz)), P::splat(-irho2));
-  const V E = P::mul(P::fma(gmgmk, cpz, P::neg(P::mul(gm1sq, cqw))), P::splat(rho));
-  const V G = P::fma(gmk, cpz, P::neg(P::mul(gm1, cqw)));
-  const V F = P::mul(P::fma(gm1sq, cpy, P::neg(P::mul(gmgmk, cqx))), P::splat(rho));
-  const V H = P::fma(gm1, cpy, P::neg(P::mul(gmk, cqx)));
+  V h, ka, kb, gmk, ngmk, rho, nrho, irho, nirho, nrho2, nirho2;
+};
+
+// One wave of a layer: cos, sin / r, -r sin (evanescent: the scaled hyperbolic
+// forms), the scale factored out and its exponent.  sin(r h) / r -> h as r -> 0.
+template <class P>
+__device__ __forceinline__ void wave32(typename P::V k, typename P::V kv, typename P::V h, typename P::V &cs,
+                                       typename P::V &sr, typename P::V &nrs, typename P::V &sc, typename P::V &ex) {
+  using V = typename P::V;
+  const V one = P::splat(1.f), half = P::splat(.5f), mhalf = P::splat(-.5f), mone = P::splat(-1.f);
+  const V X = P::mul(P::add(k, kv), P::abs(P::fma(kv, mone, k)));
+  const V ir = P::rsqrt0(X), r = P::mul(X, ir), p = P::mul(r, h);
+  V sn, cn;
+  sincos32<P>(p, &sn, &cn);
+  const V e = P::ex2(P::mul(p, P::splat(-1.4426950408889634f)));
+  const V f = P::mul(e, e);
+  const typename P::M prop = P::ltv(k, kv);
+  cs = P::sel(prop, cn, P::fma(f, half, half));
+  const V s = P::sel(prop, sn, P::fma(f, mhalf, half));
+  sr = P::sel(P::gt0(X), P::mul(s, ir), h);
+  const V t = P::mul(r, s);
+  nrs = P::sel(prop, t, P::neg(t));
+  sc = P::sel(prop, one, e);
+  ex = P::sel(prop, P::splat(0.f), p);
+}
+
+// One standard Dunkin layer step (both waves trigonometric or scaled
+// hyperbolic, selected per lane), the algebra of rayleigh_layer_f32.  Returns the
+// exponent P + Q factored out of the evanescent waves.  Signs are carried by the
+// constants (nX), by -r sin in place of r sin and by products with -1 inside a
+// multiply-add, all exact: a paired instruction has no sign of its own for an
+// operand, and flipping one takes an instruction for each half.
+template <class P>
+__device__ __forceinline__ typename P::V step32(typename P::V e[5], typename P::V k, typename P::V k2,
+                                                const Layer32<P> &l) {
+  using V = typename P::V;
+  const V mone = P::splat(-1.f), one = P::splat(1.f);
+  const V gam = P::mul(l.gmk, k2);
+  V cosp, wv, nxv, ap, xp, cosq, yv, nzv, aq, xq;
+  wave32<P>(k, l.ka, l.h, cosp, wv, nxv, ap, xp);
+  wave32<P>(k, l.kb, l.h, cosq, yv, nzv, aq, xq);
+  const V a0 = P::mul(ap, aq), expo = P::add(xp, xq);
+  const V cpcq = P::mul(cosp, cosq), cpy = P::mul(cosp, yv), ncpz = P::mul(cosp, nzv);
+  const V cqw = P::mul(cosq, wv), ncqx = P::mul(cosq, nxv);
+  const V nxy = P::mul(nxv, yv), xz = P::mul(nxv, nzv), wy = P::mul(wv, yv), nwz = P::mul(wv, nzv);
+  const V gm1 = P::add(gam, mone), ngm1 = P::fma(gam, mone, one), twgm1 = P::add(gam, gm1);
+  const V gmgmk = P::mul(gam, l.gmk), ngmgmk = P::mul(gam, l.ngmk), gm1sq = P::mul(gm1, gm1);
+  const V a0pq = P::fma(cpcq, mone, a0);
+  const V two_k2 = P::mul(k2, P::splat(2.f)), nk2 = P::mul(k2, mone);
+  V A = P::fma(P::mul(P::mul(gam, P::splat(-2.f)), gm1), a0pq, cpcq);
+  A = P::fma(ngmgmk, xz, A);
+  A = P::fma(P::mul(nk2, gm1sq), wy, A);
+  const V D = P::mul(P::fma(k2, cpy, ncqx), l.irho);
+  const V I = P::mul(P::fma(P::mul(k2, gm1), wy, P::fma(twgm1, a0pq, P::mul(l.gmk, xz))), l.nirho);
+  const V C = P::mul(P::fma(k2, cqw, ncpz), l.nirho);
+  const V Lm = P::mul(P::fma(P::mul(k2, k2), wy, P::fma(two_k2, a0pq, xz)), l.nirho2);
+  const V E = P::mul(P::fma(gmgmk, ncpz, P::mul(gm1sq, cqw)), l.nrho);
+  const V G = P::fma(l.ngmk, ncpz, P::mul(ngm1, cqw));
+  const V F = P::mul(P::fma(gm1sq, cpy, P::mul(gmgmk, ncqx)), l.rho);
+  const V H = P::fma(gm1, cpy, P::mul(l.gmk, ncqx));
   const V gg = P::mul(gmgmk, gm1sq);
   const V O = P::mul(P::fma(P::mul(gm1sq, gm1sq), wy, P::fma(P::mul(gg, P::splat(2.f)), a0pq,
                                                              P::mul(P::mul(gmgmk, gmgmk), xz))),
-                     P::splat(-rho2));
-  const V J = P::mul(P::fma(P::mul(gm1, gm1sq), wy, P::fma(P::mul(P::mul(gmk, gm1), twgm1), a0pq,
-                                                           P::mul(P::mul(gmgmk, gmk), xz))),
-                     P::splat(-rho));
-  const V K = P::fma(P::splat(2.f), P::add(cpcq, P::neg(A)), a0);
-  apply32<P>(e, k2, A, cpcq, C, D, E, F, G, H, I, J, K, Lm, P::neg(wz), P::neg(xy), O);
+                     l.nrho2);
+  const V J = P::mul(P::fma(P::mul(gm1, gm1sq), wy, P::fma(P::mul(P::mul(l.gmk, gm1), twgm1), a0pq,
+                                                           P::mul(P::mul(gmgmk, l.gmk), xz))),
+                     l.nrho);
+  const V K = P::fma(P::splat(2.f), P::fma(A, mone, cpcq), a0);
+  apply32<P>(e, k2, A, cpcq, C, D, E, F, G, H, I, J, K, Lm, nwz, nxy, O);
   return expo;
 }
 
@@ -1005,13 +1026,68 @@ __device__ __forceinline__ void start32(typename P::V e[5], typename P::V k, typ
   }
 }
 
+// Scale each lane's vector by the power of two that scale_vector takes (1 where it
+// takes none), in the lane type's own multiplications.
+template <class P>
+__device__ __forceinline__ void scale32(typename P::V e[5], int ex[P::NL]) {
+  typename P::V r;
+#pragma unroll
+  for (int i = 0; i < P::NL; ++i) {
+    float big = 0.f;
+#pragma unroll
+    for (int j = 0; j < 5; ++j) big = fmaxf(big, fabsf(lane_of(e[j], i)));
+    const bool ok = big >= 1e-30f && big < INFINITY;
+    lane_of(r, i) = ok ? pow2_inverse(big) : 1.f;
+    ex[i] += ok ? binade(big) : 0;
+  }
+#pragma unroll
+  for (int j = 0; j < 5; ++j) e[j] = P::mul(e[j], r);
+}
+
+// The layers of a model as the evaluations read them: R1 from the model's table,
+// R2 from its records of PAIR_ROW float pairs a layer (each constant twice, negated
+// where step32 wants it so: six 16-byte loads and no moves or sign flips).
+constexpr int PAIR_ROW = 12;
+enum PairRow { PR_H = 0, PR_IVP, PR_IVS, PR_VS2, PR_NVS2, PR_RHO, PR_NRHO, PR_IRHO, PR_NIRHO, PR_NRHO2, PR_NIRHO2 };
+struct Layers1 {
+  LayerView<float> m;
+  __device__ __forceinline__ Layer32<R1> get(int l, float w, float iw2, float &ivp, float &ivs) const {
+    const float vs2 = m.vs2(l), rho = m.rho(l), irho = m.irho(l);
+    ivp = m.ivp(l);
+    ivs = m.ivs(l);
+    const float g = x_mul(x_mul(iw2, vs2), 2.f);
+    return {m.h(l), x_mul(w, ivp), x_mul(w, ivs), g, -g, rho, -rho, irho, -irho, -x_mul(rho, rho), -x_mul(irho, irho)};
+  }
+};
+struct Layers2 {
+  LayerView<float> m;
+  const float4 *rec;
+  __device__ __forceinline__ Layer32<R2> get(int l, float w, float iw2, float &ivp, float &ivs) const {
+    const float4 *r = rec + static_cast<size_t>(l) * (PAIR_ROW / 2);
+    const float4 q0 = r[0], q1 = r[1], q2 = r[2], q3 = r[3], q4 = r[4], q5 = r[5];
+    const float2 ww = make_float2(w, w), ii = make_float2(iw2, iw2);
+    auto lo = [](const float4 &q) { return make_float2(q.x, q.y); };
+    auto hi = [](const float4 &q) { return make_float2(q.z, q.w); };
+    ivp = q0.z;
+    ivs = q1.x;
+    // (twice vs^2 in the record: the same value as twice the product)
+    return {lo(q0), R2::mul(ww, hi(q0)), R2::mul(ww, lo(q1)), R2::mul(ii, hi(q1)), R2::mul(ii, lo(q2)),
+            hi(q2), lo(q3), hi(q3), lo(q4), hi(q4), lo(q5)};
+  }
+};
+template <class P> struct Layers32;
+template <> struct Layers32<R1> { using type = Layers1; };
+template <> struct Layers32<R2> { using type = Layers2; };
+
 // Rayleigh secular value, shape feature and base-2 log-magnitude of one (R1) or
 // two (R2) samples of one trace at frequency w: the single-precision path of
 // rayleigh_multi, explicitly rounded.  c holds the samples' velocities w / k.
 template <class P>
-__device__ __forceinline__ void rayleigh_eval32(const LayerView<float> &m, typename P::V k, typename P::V c, float w,
-                                                typename P::V *F, typename P::V *shape, typename P::V *lmag) {
+__device__ __forceinline__ void rayleigh_eval32(const typename Layers32<P>::type &layers, typename P::V k,
+                                                typename P::V c, float w, typename P::V *F, typename P::V *shape,
+                                                typename P::V *lmag) {
   using V = typename P::V;
+  const LayerView<float> &m = layers.m;
   constexpr int NL = P::NL;
   const float tiny = 1e-30f;
   const float iw = 1.f / w, iw2 = x_mul(iw, iw);
@@ -1019,55 +1095,45 @@ __device__ __forceinline__ void rayleigh_eval32(const LayerView<float> &m, typen
   const V k2 = P::mul(k, k);
   V e[5];
   start32<P>(e, k, k2, c, w, iw2, m.ivp(last), m.ivs(last), m.vs2(last), m.rho(last));
-  int ex[NL];
+  int ex[NL] = {};
   V ev = P::splat(0.f);
+  scale32<P>(e, ex);
+  // the lowest of the lanes' velocities decides whether any takes the factored step
+  float cl = lane_of(c, 0);
 #pragma unroll
-  for (int i = 0; i < NL; ++i) {
-    float t[5] = {lane_of(e[0], i), lane_of(e[1], i), lane_of(e[2], i), lane_of(e[3], i), lane_of(e[4], i)};
-    ex[i] = scale_vector(t, 5, tiny);
-#pragma unroll
-    for (int j = 0; j < 5; ++j) lane_of(e[j], i) = t[j];
-  }
+  for (int i = 1; i < NL; ++i) cl = fminf(cl, lane_of(c, i));
+  cl = x_mul(MD200_EVANESCENT_RATIO, cl);
   for (int l = m.L - 2; l >= m.water; --l) {
-    const float h = m.h(l), ivp = m.ivp(l), vs2 = m.vs2(l), ivs = m.ivs(l), rho = m.rho(l), irho = m.irho(l);
-    const float ka = x_mul(w, ivp), kb = x_mul(w, ivs), gammk = x_mul(x_mul(iw2, vs2), 2.f);
-    const float rho2 = x_mul(rho, rho), irho2 = x_mul(irho, irho);
-    bool evan[NL], any = false, all = true;
-#pragma unroll
-    for (int i = 0; i < NL; ++i) {
-      evan[i] = x_mul(x_mul(MD200_EVANESCENT_RATIO, lane_of(c, i)), ivs) < 1.f;
-      any |= evan[i];
-      all &= evan[i];
-    }
-    V en[5] = {e[0], e[1], e[2], e[3], e[4]};
+    float ivp, ivs;
+    const Layer32<P> ly = layers.get(l, w, iw2, ivp, ivs);
     V expo = P::splat(0.f);
-    if constexpr (NL == 1) {
-      if (evan[0]) expo = evanescent32(en, k, k2, c, h, ivp, ivs, rho, irho, rho2, irho2);
-      else expo = step32<P>(en, k, k2, ka, kb, gammk, h, rho, irho, rho2, irho2);
+    if (!(x_mul(cl, ivs) < 1.f)) {
+      expo = step32<P>(e, k, k2, ly);
     } else {
-      if (!all) expo = step32<P>(en, k, k2, ka, kb, gammk, h, rho, irho, rho2, irho2);
-      if (any) {
+      V en[5] = {e[0], e[1], e[2], e[3], e[4]};
+      bool evan[NL], all = true;
 #pragma unroll
-        for (int i = 0; i < NL; ++i) {
-          if (evan[i]) {
-            float t[5] = {lane_of(e[0], i), lane_of(e[1], i), lane_of(e[2], i), lane_of(e[3], i),
-                          lane_of(e[4], i)};
-            lane_of(expo, i) = evanescent32(t, lane_of(k, i), lane_of(k2, i), lane_of(c, i), h, ivp, ivs, rho,
-                                            irho, rho2, irho2);
+      for (int i = 0; i < NL; ++i) {
+        evan[i] = x_mul(x_mul(MD200_EVANESCENT_RATIO, lane_of(c, i)), ivs) < 1.f;
+        all &= evan[i];
+      }
+      if (!all) expo = step32<P>(en, k, k2, ly);
 #pragma unroll
-            for (int j = 0; j < 5; ++j) lane_of(en[j], i) = t[j];
-          }
+      for (int i = 0; i < NL; ++i) {
+        if (evan[i]) {
+          float t[5] = {lane_of(e[0], i), lane_of(e[1], i), lane_of(e[2], i), lane_of(e[3], i), lane_of(e[4], i)};
+          lane_of(expo, i) = evanescent32(t, lane_of(k, i), lane_of(k2, i), lane_of(c, i), lane_of(ly.h, 0), ivp, ivs,
+                                          lane_of(ly.rho, 0), lane_of(ly.irho, 0), -lane_of(ly.nrho2, 0),
+                                          -lane_of(ly.nirho2, 0));
+#pragma unroll
+          for (int j = 0; j < 5; ++j) lane_of(en[j], i) = t[j];
         }
       }
+#pragma unroll
+      for (int j = 0; j < 5; ++j) e[j] = en[j];
     }
     ev = P::add(ev, expo);
-#pragma unroll
-    for (int i = 0; i < NL; ++i) {
-      float t[5] = {lane_of(en[0], i), lane_of(en[1], i), lane_of(en[2], i), lane_of(en[3], i), lane_of(en[4], i)};
-      ex[i] += scale_vector(t, 5, tiny);
-#pragma unroll
-      for (int j = 0; j < 5; ++j) lane_of(e[j], i) = t[j];
-    }
+    scale32<P>(e, ex);
   }
   V lm;
 #pragma unroll
@@ -1133,7 +1199,7 @@ MD200_FN void rayleigh_multi(const LayerView<T> &m, const N *k, const N &w, N *F
   // the scan's single-precision evaluations: explicitly rounded (rayleigh_eval32)
   if constexpr (std::is_same<N, float>::value && std::is_same<T, float>::value && S == 1) {
     if (levan == nullptr && fmax == nullptr) {
-      rayleigh_eval32<R1>(m, k[0], w / k[0], w, F, shape, lmag);
+      rayleigh_eval32<R1>(Layers1{m}, k[0], w / k[0], w, F, shape, lmag);
       return;
     }
   }

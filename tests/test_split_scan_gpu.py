@@ -137,3 +137,20 @@ def test_split_equals_fused_beyond_one_active_set():
     split = solve(batch, periods, 5, 0, SPLIT)
     fused = solve(batch, periods, 5, 0, FUSED)
     assert_identical(split, fused, "beyond one active set")
+
+
+@pytest.mark.parametrize("rows", [2, 55, 56, 57, 60, 256])
+def test_split_equals_fused_over_row_counts(rows):
+    """The staged layer records: one and two buffers, rows that fill a record block or leave a rest."""
+    rng = np.random.default_rng(rows)
+    B = 24
+    vs = np.sort(rng.uniform(.5, 4., (B, rows)), axis=1)
+    vs[:, -1] = 4.2
+    vp = vs * rng.uniform(1.7, 2., (B, rows))
+    h = rng.uniform(20., 60., (B, rows)) / rows
+    h[:, -1] = 0.
+    if rows > 2:
+        h[::3, rows // 2:-1] = 0.  # shorter stacks in the same batch
+    batch = dict(thickness=h, vp=vp, vs=vs, rho=1.74 * vp ** .25)
+    periods = np.geomspace(.5, 40., 23)
+    assert_identical(solve(batch, periods, 4, 0, FUSED), solve(batch, periods, 4, 0, SPLIT), f"{rows} rows")
