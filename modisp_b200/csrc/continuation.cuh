@@ -218,7 +218,7 @@ __device__ __noinline__ double cont_eval(const LayerView<double> m, int wave, do
   return secular<double, double>(m, wave, w / c, w, g);
 }
 __device__ __noinline__ RootSample cont_sample(const LayerView<double> m, int wave, double w, double c) {
-  return root_sample(m, wave, w, c);
+  return wave ? root_sample<1>(m, w, c) : root_sample<0>(m, w, c);
 }
 
 // ---------------------------------------------------------------------------

@@ -496,6 +496,7 @@ int enqueue(md200_engine *e, const double *h, const double *vp, const double *vs
   Dev dm = d;
   dm.model_lists = nt >= MODEL_LIST_MIN_TRACES ? 1 : 0;
   const int model_blocks = (B + 3) / 4;
+  const auto refine_fn = wave == 0 ? refine<0> : refine<1>;
   const bool split = d.fp32 && (e->o.scan_mode == 2 ||
                                 (e->o.scan_mode == 0 && wave == 0 && nt >= SPLIT_MIN_TRACES));
   if (split) {
@@ -519,7 +520,7 @@ int enqueue(md200_engine *e, const double *h, const double *vp, const double *vs
     list_brackets<<<model_blocks, 128, 0, s>>>(d);
     ++nl;
   }
-  refine<<<e->list_blocks, 128, 0, s>>>(d);
+  refine_fn<<<e->list_blocks, 128, 0, s>>>(d);
   ++nl;
   MD200_CK(cudaGetLastError());
   MD200_CK(mark(4));
@@ -535,7 +536,7 @@ int enqueue(md200_engine *e, const double *h, const double *vp, const double *vs
                                                                                  C_REPAIR_CURSOR, C_NREPAIR);
     ++nl;
     MD200_CK(mark(6));
-    refine<<<e->list_blocks, 128, 0, s>>>(d);
+    refine_fn<<<e->list_blocks, 128, 0, s>>>(d);
     ++nl;
     MD200_CK(cudaGetLastError());
   } else {
@@ -573,7 +574,7 @@ int enqueue(md200_engine *e, const double *h, const double *vp, const double *vs
                                                                                  C_REPAIR_CURSOR, C_NREPAIR);
     ++nl;
     MD200_CK(cudaGetLastError());
-    refine<<<e->list_blocks, 128, 0, s>>>(d);
+    refine_fn<<<e->list_blocks, 128, 0, s>>>(d);
     ++nl;
     assemble<<<(nt + 255) / 256, 256, 0, s>>>(d, d.repair_list, C_NREPAIR);
     ++nl;
@@ -605,7 +606,7 @@ int enqueue(md200_engine *e, const double *h, const double *vp, const double *vs
       scan<double, 1><<<e->scan_blocks64, 32 * e->scan_warps, e->scan_smem64, s>>>(d, d.repair_list,
                                                                                  C_REPAIR_CURSOR, C_NREPAIR);
     ++nl;
-    refine<<<e->list_blocks, 128, 0, s>>>(d);
+    refine_fn<<<e->list_blocks, 128, 0, s>>>(d);
     ++nl;
     assemble<<<(nt + 255) / 256, 256, 0, s>>>(d, d.cont_list, C_NTARGET);
     ++nl;
@@ -632,7 +633,7 @@ int enqueue(md200_engine *e, const double *h, const double *vp, const double *vs
                                                                                  C_REPAIR_CURSOR, C_NREPAIR);
     ++nl;
     MD200_CK(cudaGetLastError());
-    refine<<<e->list_blocks, 128, 0, s>>>(d);
+    refine_fn<<<e->list_blocks, 128, 0, s>>>(d);
     ++nl;
     assemble<<<(nt + 255) / 256, 256, 0, s>>>(d, d.repair_list, C_NREPAIR);
     ++nl;
@@ -1325,7 +1326,7 @@ int md200_kernel_report(int layers, int single_precision, char *json, int length
       {"scan_fp32", reinterpret_cast<const void *>(scan<float, 0>)},
       {"scan_fp64_love", reinterpret_cast<const void *>(scan<double, 1>)},
       {"scan_fp32_love", reinterpret_cast<const void *>(scan<float, 1>)},
-      {"refine", reinterpret_cast<const void *>(refine)},
+      {"refine", reinterpret_cast<const void *>(refine<0>)},
       {"assemble", reinterpret_cast<const void *>(assemble)},
       {"group_velocity", reinterpret_cast<const void *>(group_velocity)},
   };

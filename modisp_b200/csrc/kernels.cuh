@@ -1302,10 +1302,11 @@ __device__ __forceinline__ double sample_ratio(const RootSample &x, const RootSa
   const double dl = x.l - y.l;
   return isnan(dl) ? x.F / y.F : (x.g / y.g) * exp2(dl);
 }
-__device__ __forceinline__ RootSample root_sample(const LayerView<double> &m, int wave, double w, double c) {
+template <int WAVE>
+__device__ __forceinline__ RootSample root_sample(const LayerView<double> &m, double w, double c) {
   RootSample r;
   double lev;
-  r.F = secular<double, double>(m, wave, w / c, w, &r.g, &r.l, &lev);
+  r.F = secular<double, double>(m, WAVE, w / c, w, &r.g, &r.l, &lev);
   r.l -= lev;
   return r;
 }
@@ -1593,6 +1594,7 @@ __device__ __forceinline__ void refine_fetch(Dev &d, RefineLane &L, int end, int
 #ifndef MD200_REFINE_MIN_BLOCKS
 #define MD200_REFINE_MIN_BLOCKS 4
 #endif
+template <int WAVE>
 __global__ void __launch_bounds__(128, MD200_REFINE_MIN_BLOCKS) refine(Dev d) {
   const int lane = threadIdx.x & 31;
   const int end = d.ctr[C_NREFINE];
@@ -1607,14 +1609,16 @@ __global__ void __launch_bounds__(128, MD200_REFINE_MIN_BLOCKS) refine(Dev d) {
   for (;;) {
     double x = 0.;
     L.eval = false;
-    refine_step(d, L, &x, count);
-    refine_fetch(d, L, end, chunk, lane);
-    refine_step(d, L, &x, count);
-    refine_fetch(d, L, end, chunk, lane);
-    refine_step(d, L, &x, count);
+    // (a loop, and one wave a kernel: the instruction cache missed twice an issue)
+#pragma unroll 1
+    for (int pass = 0;; ++pass) {
+      refine_step(d, L, &x, count);
+      if (pass == 2 || __all_sync(FULL, L.eval || L.exhausted)) break;
+      refine_fetch(d, L, end, chunk, lane);
+    }
     if (__all_sync(FULL, !L.eval && L.exhausted)) break;
     if (L.eval) {
-      const RootSample smp = root_sample(L.m, d.wave, L.w, x);  // the one evaluation site
+      const RootSample smp = root_sample<WAVE>(L.m, L.w, x);  // the one evaluation site
       brent_absorb(L.st, smp);
       ++evals;
       steps += layer_steps(L.m.L, L.m.water);
