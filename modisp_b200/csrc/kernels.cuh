@@ -562,15 +562,88 @@ __global__ void tail_values(Dev d) {
   }
 }
 
-// Position of scan point j (1 <= j <= J) of a trace: invert
-// u(c) = f N(c) + alpha ln c at u_lo + j / density through the knot table.  In
-// an interval that starts at a body velocity the kink term grows like
+// Index (0..32) of the first lane whose sorted value is >= x (or > x when
+// `inclusive`), over the warp's ascending per-lane values `v`.
+__device__ __forceinline__ int warp_rank(double v, double x, bool inclusive) {
+  int lo = 0, hi = 32;
+#pragma unroll
+  for (int it = 0; it < 6; ++it) {
+    const int mid = (lo + hi) >> 1;
+    const double m = __shfl_sync(FULL, v, mid & 31);
+    const bool less = inclusive ? (m <= x) : (m < x);
+    if (lo < hi) {
+      if (less) lo = mid + 1; else hi = mid;
+    }
+  }
+  return lo;
+}
+
+// The position at u = target in the knot interval [x0, x1], u0 = u(x0), u1 = u(x1),
+// `kink` the part of u1 - u0 that grows like a square root.
+__device__ __forceinline__ double knot_position(double target, double u0, double u1, double x0, double x1,
+                                                double kink) {
+  // the fractional position within the knot interval needs only single precision
+  const float dt = static_cast<float>(fmax(0., target - u0)), du = static_cast<float>(u1 - u0);
+  const float a = static_cast<float>(kink), bs = fmaxf(0.f, du - a);
+  float s = 0.f;
+  if (du > 0.f && dt > 0.f) {  // (dt = 0 would give 0/0 where the interval has no kink)
+    const float x = 2.f * dt / (a + sqrtf(a * a + 4.f * bs * dt));
+    s = fminf(1.f, x * x);
+  }
+  return fma(x1 - x0, static_cast<double>(s), x0);
+}
+
+// Positions of 32 scan points of a trace, one per lane (targets ascending with the
+// lane; +INFINITY: no point): invert u(c) = f N(c) + alpha ln c through the knot
+// table.  In an interval that starts at a body velocity the kink term grows like
 // sqrt(c - c_i); the local model u = u_i + a sqrt(s) + b s (s the fractional
 // position) is inverted exactly.
 //
-// `from` is a knot index at or below the interval of `target` (each lane's
-// targets increase from step to step, so the lane's previous interval
-// qualifies): the interval is found by galloping up from it and bisecting the
+// The warp reads 32 knots at a time, from `from` on (a knot at or below the first
+// target's interval), and every lane finds its interval -- the last knot with
+// u <= target -- by a binary search over the lanes' values: a coalesced load or two
+// where each lane walking the table on its own waits for some ten dependent ones
+// (scan_point).  32 points span about as many knots.  Scan stage of 20,000
+// low-velocity-layer models x 60 periods: Love FP32 21.1 -> 19.7 ms, FP64 34.3 ->
+// 32.4; the split Rayleigh scan 39.2 -> 38.6.  On return `iv` holds the lane's interval.
+__device__ __forceinline__ double scan_points32(const double4 *kt, int nk, double f, double alpha, double target,
+                                                int from, int lane, int &iv) {
+  const bool wanted = target < INFINITY;
+  bool found = !wanted;
+  double u0 = 0., u1 = 1., x0 = 0., x1 = 0., kink = 0.;
+  iv = from;
+  for (int base = from;; base = min(base + 31, nk - 2)) {
+    const int j = base + lane;
+    double4 q = make_double4(0., 0., 0., 0.);
+    double u = INFINITY;
+    if (j < nk) {
+      q = kt[j];
+      u = fma(f, q.y, alpha * q.z);
+    }
+    const int n = warp_rank(u, target, true);  // knots of this batch at or below the target
+    const bool here = !found && n < 32;
+    const int l = max(0, min(n - 1, nk - 2 - base));
+    const double a0 = __shfl_sync(FULL, u, l), a1 = __shfl_sync(FULL, u, l + 1);
+    const double b0 = __shfl_sync(FULL, q.x, l), b1 = __shfl_sync(FULL, q.x, l + 1);
+    const double w0 = __shfl_sync(FULL, q.w, l);
+    if (here) {
+      u0 = a0;
+      u1 = a1;
+      x0 = b0;
+      x1 = b1;
+      kink = w0;
+      iv = base + l;
+      found = true;
+    }
+    if (__all_sync(FULL, found)) break;
+  }
+  return wanted ? knot_position(target, u0, u1, x0, x1, f * kink) : INFINITY;
+}
+
+// Position of one scan point, the same inversion by one lane on its own (the FP64
+// Rayleigh scan: FP64-pipe bound, 81.3 ms with this search and 84.6 ms with the
+// warp's).  `from` is a knot index at or below the interval of `target` (each lane's targets
+// increase from step to step, so the lane's previous interval qualifies): the interval is found by galloping up from it and bisecting the
 // last gap -- the same interval a bisection of the whole table finds (the last
 // knot with u <= target), in a few table reads instead of ~8 dependent ones.
 // On return `from` holds that interval.
@@ -592,32 +665,7 @@ __device__ __forceinline__ double scan_point(const double4 *kt, int nk, double f
   }
   from = lo;
   const double4 q0 = kt[lo], q1 = kt[hi];
-  const double u0 = fma(f, q0.y, alpha * q0.z), u1 = fma(f, q1.y, alpha * q1.z);
-  // the fractional position within the knot interval needs only single precision
-  const float dt = static_cast<float>(fmax(0., target - u0)), du = static_cast<float>(u1 - u0);
-  const float a = static_cast<float>(f * q0.w), bs = fmaxf(0.f, du - a);
-  float s = 0.f;
-  if (du > 0.f && dt > 0.f) {  // (dt = 0 would give 0/0 where the interval has no kink)
-    const float x = 2.f * dt / (a + sqrtf(a * a + 4.f * bs * dt));
-    s = fminf(1.f, x * x);
-  }
-  return fma(q1.x - q0.x, static_cast<double>(s), q0.x);
-}
-
-// Index (0..32) of the first lane whose sorted value is >= x (or > x when
-// `inclusive`), over the warp's ascending per-lane values `v`.
-__device__ __forceinline__ int warp_rank(double v, double x, bool inclusive) {
-  int lo = 0, hi = 32;
-#pragma unroll
-  for (int it = 0; it < 6; ++it) {
-    const int mid = (lo + hi) >> 1;
-    const double m = __shfl_sync(FULL, v, mid & 31);
-    const bool less = inclusive ? (m <= x) : (m < x);
-    if (lo < hi) {
-      if (less) lo = mid + 1; else hi = mid;
-    }
-  }
-  return lo;
+  return knot_position(target, fma(f, q0.y, alpha * q0.z), fma(f, q1.y, alpha * q1.z), q0.x, q1.x, f * q0.w);
 }
 
 // Global-memory FP64 view of model b.
@@ -958,15 +1006,23 @@ __device__ __forceinline__ ScanState scan_start(const Dev &d, const TraceCtx &x)
 // The next 32 sample positions: grid points and seeds merged in order (this
 // lane's position in c; INFINITY past the window).  Returns the valid-lane mask;
 // with SRC, also (*seeds) the lanes whose position is a seed (kbuf: 32 bytes of
-// shared memory beside mbuf).
-template <bool SRC = false>
+// shared memory beside mbuf) and (*kfirst) the first grid point's knot interval.
+// kfrom: a knot at or below the next grid point's interval, moved along.
+template <bool SRC = false, bool WARP_SEARCH = true>
 __device__ __forceinline__ unsigned scan_positions(const TraceCtx &x, ScanState &st, double step, int lane,
                                                    double *mbuf, int &kfrom, double &c,
-                                                   unsigned char *kbuf = nullptr, unsigned *seeds = nullptr) {
+                                                   unsigned char *kbuf = nullptr, unsigned *seeds = nullptr,
+                                                   int *kfirst = nullptr) {
   const long long gj = st.gi + lane;
-  const double gv = gj <= st.J ? scan_point(x.kt, x.nk, x.fr, x.alpha, x.u_lo + static_cast<double>(gj) * step,
-                                            kfrom)
-                               : INFINITY;
+  const double target = gj <= st.J ? x.u_lo + static_cast<double>(gj) * step : INFINITY;
+  int iv = kfrom;
+  double gv = INFINITY;
+  if constexpr (WARP_SEARCH) {
+    if (st.gi <= st.J) gv = scan_points32(x.kt, x.nk, x.fr, x.alpha, target, kfrom, lane, iv);
+  } else {
+    if (gj <= st.J) gv = scan_point(x.kt, x.nk, x.fr, x.alpha, target, kfrom);
+  }
+  if constexpr (SRC) *kfirst = __shfl_sync(FULL, iv, 0);
   double sv = st.si + lane < x.ns ? x.sd[st.si + lane] : INFINITY;
   if ((st.tfl & TRACE_WORKSPACE_LIMIT) && st.gi + 31 >= st.J) {
     // a capped grid ends in this step (or has ended): seeds past its last point
@@ -983,6 +1039,7 @@ __device__ __forceinline__ unsigned scan_positions(const TraceCtx &x, ScanState 
     c = gv;
     if constexpr (SRC) *seeds = 0u;
     st.gi += 32;
+    if constexpr (WARP_SEARCH) kfrom = __shfl_sync(FULL, iv, 31);
     return FULL;
   }
   const int rg = warp_rank(sv, gv, false);  // seeds strictly below this scan point
@@ -1000,7 +1057,9 @@ __device__ __forceinline__ unsigned scan_positions(const TraceCtx &x, ScanState 
   c = mbuf[lane];
   if constexpr (SRC) *seeds = __ballot_sync(FULL, c < INFINITY && kbuf[lane]);
   __syncwarp();
-  st.gi += __popc(__ballot_sync(FULL, pg < 32 && gv < INFINITY));
+  const int taken = __popc(__ballot_sync(FULL, pg < 32 && gv < INFINITY));
+  st.gi += taken;
+  if constexpr (WARP_SEARCH) kfrom = __shfl_sync(FULL, iv, min(taken, 31));  // the first point not taken lies at or above
   st.si += __popc(__ballot_sync(FULL, ps < 32 && sv < INFINITY));
   return __ballot_sync(FULL, c < INFINITY);
 }
@@ -1241,12 +1300,12 @@ __global__ void __launch_bounds__(128, (sizeof(T) == 4 && WAVE == 1) ? MD200_SCA
     else view64 = *reinterpret_cast<const LayerView<double> *>(&view);
     // a fresh trace, or (resume) one the split scan handed over mid-way
     ScanState st = resume ? d.sp_state[x.t] : scan_start(d, x);
-    // this lane's knot interval (scan_point): below the first grid point every
+    // the knot interval scan_points32 starts from: below the first grid point every
     // knot is a log point
     int kfrom = resume ? 0 : max(0, static_cast<int>(st.gi) - 2);
     while (st.nbr < x.K && !(st.bits & SS_FINISHED)) {
       double c;
-      const unsigned vm = scan_positions(x, st, step, lane, mbuf, kfrom, c);
+      const unsigned vm = scan_positions<false, single || WAVE == 1>(x, st, step, lane, mbuf, kfrom, c);
       if (!vm) {
         st.bits |= SS_FINISHED;  // the window is exhausted
         break;

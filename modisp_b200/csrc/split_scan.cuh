@@ -186,9 +186,10 @@ __global__ void __launch_bounds__(128) split_positions(Dev d, int p) {
       double c = INFINITY;
       unsigned seeds = 0;
       if (!done) {
-        const unsigned vm = scan_positions<true>(x, st, step, lane, mbuf, kfrom, c, kbuf, &seeds);
+        int kfirst;
+        const unsigned vm = scan_positions<true>(x, st, step, lane, mbuf, kfrom, c, kbuf, &seeds, &kfirst);
         done = vm == 0;
-        if (s == 0 && lane == 0) d.sp_kf[t] = kfrom;
+        if (s == 0 && lane == 0) d.sp_kf[t] = kfirst;
       }
       unsigned k = 0;
       if (c < INFINITY) {
