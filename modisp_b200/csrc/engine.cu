@@ -316,8 +316,10 @@ int setup(md200_engine *e, bool staging) {
   for (auto fn : {scan<float, 0>, scan<float, 1>})
     MD200_CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   static_cast<int>(std::max<size_t>(e->scan_smem32, 1024))));
-  MD200_CK(cudaFuncSetAttribute(split_eval32_pair, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                static_cast<int>(split_pair_smem(d.Ls, split_pair_buffers(d.Ls)))));
+  MD200_CK(cudaFuncSetAttribute(split_eval32_pair<0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                static_cast<int>(split_pair_smem(0, d.Ls, split_pair_buffers(0, d.Ls)))));
+  MD200_CK(cudaFuncSetAttribute(split_eval32_pair<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                static_cast<int>(split_pair_smem(1, d.Ls, split_pair_buffers(1, d.Ls)))));
   int occ64 = 0, occ32 = 0;
   MD200_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ64, scan<double, 0>, 32 * e->scan_warps,
                                                          e->scan_smem64));
@@ -391,7 +393,7 @@ int split_scan(md200_engine *e, const Dev &d, int rounds, cudaStream_t s) {
   const int cap = d.sp_cap;
   const int fill_blocks = std::max(1, std::min((cap + 255) / 256, sms * 8));
   const int pos_blocks = std::max(1, std::min((cap + 3) / 4, sms * 16));
-  const int eval_blocks = sms * 16, buffers = split_pair_buffers(d.Ls);
+  const int buffers = split_pair_buffers(WAVE, d.Ls);
   const int book_blocks = std::max(1, std::min((cap + 127) / 128, sms * 8));
   int nl = 0;
   for (int r = 0; r < rounds; ++r) {
@@ -401,15 +403,15 @@ int split_scan(md200_engine *e, const Dev &d, int rounds, cudaStream_t s) {
     split_positions<<<pos_blocks, 128, 0, s>>>(d, p);
     if (!e->capturing && cudaEventRecord(e->sp_ev[2 * r], s) != cudaSuccess) return -1;
 #if MD200_SPLIT_PAIR
-    if (WAVE == 0)
-      split_eval32_pair<<<sms * MD200_SPLIT_PAIR_GRID, 128, split_pair_smem(d.Ls, buffers), s>>>(d, p, buffers);
-    else
+    split_eval32_pair<WAVE>
+        <<<sms * MD200_SPLIT_PAIR_GRID, 128, split_pair_smem(WAVE, d.Ls, buffers), s>>>(d, p, buffers);
+#else
+    split_eval32<WAVE><<<sms * 16, 128, 0, s>>>(d, p);
 #endif
-      split_eval32<WAVE><<<eval_blocks, 128, 0, s>>>(d, p);
     if (!e->capturing && cudaEventRecord(e->sp_ev[2 * r + 1], s) != cudaSuccess) return -1;
     split_redo<WAVE><<<sms * 8, 128, 0, s>>>(d, p);
     split_book<WAVE><<<book_blocks, 128, 0, s>>>(d, p);
-    split_zoom<WAVE><<<sms * 4, 128, 0, s>>>(d, p);
+    split_zoom<WAVE><<<sms * 8, 128, 0, s>>>(d, p);
     nl += 7;
   }
   e->sp_timed = e->capturing ? 0 : rounds;

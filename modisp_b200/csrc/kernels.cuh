@@ -265,15 +265,19 @@ __global__ void prep_models(Dev d, int sortcap, int automatic) {
         t64[q * Ls + r] = vals[q];
         t32[q * Ls + r] = static_cast<float>(vals[q]);
       }
-      if (d.fp32 && !d.wave) {  // the paired evaluation's record of this layer
+      if (d.fp32) {  // the paired evaluation's record of this layer
         const float h = static_cast<float>(vals[0]), vs2 = static_cast<float>(vals[3]), rho = static_cast<float>(vals[4]);
         const float irho = static_cast<float>(vals[5]), nrho2 = -x_mul(rho, rho), nirho2 = -x_mul(irho, irho);
         const float rec[PAIR_ROW] = {h,    static_cast<float>(vals[1]), static_cast<float>(vals[2]),
                                      2.f * vs2, -2.f * vs2, rho, -rho, irho, -irho, nrho2, nirho2, 0.f};
-        float4 *out = reinterpret_cast<float4 *>(d.pair32 + (static_cast<size_t>(b) * Ls + r) * PAIR_ROW * 2);
+        const float love[PAIR_ROW_LOVE] = {h, static_cast<float>(vals[2]), x_mul(rho, vs2), static_cast<float>(vals[6])};
+        const int row = pair_row(d.wave);
+        float4 *out = reinterpret_cast<float4 *>(d.pair32) + (static_cast<size_t>(b) * Ls + r) * (row / 2);
 #pragma unroll
-        for (int q = 0; q < PAIR_ROW / 2; ++q)
-          out[q] = make_float4(rec[2 * q], rec[2 * q], rec[2 * q + 1], rec[2 * q + 1]);
+        for (int q = 0; q < PAIR_ROW / 2; ++q) {
+          if (!d.wave) out[q] = make_float4(rec[2 * q], rec[2 * q], rec[2 * q + 1], rec[2 * q + 1]);
+          else if (q < PAIR_ROW_LOVE / 2) out[q] = make_float4(love[2 * q], love[2 * q], love[2 * q + 1], love[2 * q + 1]);
+        }
       }
     }
     L += __popc(mask);

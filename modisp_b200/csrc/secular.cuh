@@ -1028,27 +1028,28 @@ __device__ __forceinline__ void start32(typename P::V e[5], typename P::V k, typ
 
 // Scale each lane's vector by the power of two that scale_vector takes (1 where it
 // takes none), in the lane type's own multiplications.
-template <class P>
-__device__ __forceinline__ void scale32(typename P::V e[5], int ex[P::NL]) {
+template <class P, int N>
+__device__ __forceinline__ void scale32(typename P::V (&e)[N], int (&ex)[P::NL]) {
   typename P::V r;
 #pragma unroll
   for (int i = 0; i < P::NL; ++i) {
     float big = 0.f;
 #pragma unroll
-    for (int j = 0; j < 5; ++j) big = fmaxf(big, fabsf(lane_of(e[j], i)));
+    for (int j = 0; j < N; ++j) big = fmaxf(big, fabsf(lane_of(e[j], i)));
     const bool ok = big >= 1e-30f && big < INFINITY;
     lane_of(r, i) = ok ? pow2_inverse(big) : 1.f;
     ex[i] += ok ? binade(big) : 0;
   }
 #pragma unroll
-  for (int j = 0; j < 5; ++j) e[j] = P::mul(e[j], r);
+  for (int j = 0; j < N; ++j) e[j] = P::mul(e[j], r);
 }
 
 // The layers of a model as the evaluations read them: R1 from the model's table,
 // R2 from its records of PAIR_ROW float pairs a layer (each constant twice, negated
 // where step32 wants it so: six 16-byte loads and no moves or sign flips).
-constexpr int PAIR_ROW = 12;
-enum PairRow { PR_H = 0, PR_IVP, PR_IVS, PR_VS2, PR_NVS2, PR_RHO, PR_NRHO, PR_IRHO, PR_NIRHO, PR_NRHO2, PR_NIRHO2 };
+// Love: h, 1/vs, mu, 1/mu.
+constexpr int PAIR_ROW = 12, PAIR_ROW_LOVE = 4;
+__host__ __device__ constexpr int pair_row(int wave) { return wave ? PAIR_ROW_LOVE : PAIR_ROW; }
 struct Layers1 {
   LayerView<float> m;
   __device__ __forceinline__ Layer32<R1> get(int l, float w, float iw2, float &ivp, float &ivs) const {
@@ -1300,11 +1301,98 @@ MD200_FN typename Base<N>::type love_entries(const N &k, const N &kj, T h, N *cq
   return wave_block<N, T>(k, kj, h, cq, y, z, &scale);
 }
 
+#if defined(__CUDACC__)
+// The layers of a model for the single-precision Love evaluations: R1 from the
+// model's table, R2 from its records of PAIR_ROW_LOVE float pairs.
+template <class P>
+struct LoveLayer32 {
+  typename P::V h, kj, mu, imu;
+};
+struct Love1 {
+  LayerView<float> m;
+  __device__ __forceinline__ LoveLayer32<R1> get(int l, float w) const {
+    return {m.h(l), x_mul(w, m.ivs(l)), x_mul(m.rho(l), m.vs2(l)), m.imu(l)};
+  }
+};
+struct Love2 {
+  LayerView<float> m;
+  const float4 *rec;
+  __device__ __forceinline__ LoveLayer32<R2> get(int l, float w) const {
+    const float4 q0 = rec[2 * l], q1 = rec[2 * l + 1];
+    return {make_float2(q0.x, q0.y), R2::mul(make_float2(w, w), make_float2(q0.z, q0.w)), make_float2(q1.x, q1.y),
+            make_float2(q1.z, q1.w)};
+  }
+};
+template <class P> struct LoveLayers32;
+template <> struct LoveLayers32<R1> { using type = Love1; };
+template <> struct LoveLayers32<R2> { using type = Love2; };
+
+// Love secular value, shape feature and base-2 log-magnitude of one (R1) or two
+// (R2) samples of one trace: the single-precision path of love_multi, explicitly
+// rounded as rayleigh_eval32 is, so that paired and single evaluations agree bit
+// for bit.
+template <class P>
+__device__ __forceinline__ void love_eval32(const typename LoveLayers32<P>::type &layers, typename P::V k, float w,
+                                            typename P::V *F, typename P::V *shape, typename P::V *lmag) {
+  using V = typename P::V;
+  const LayerView<float> &m = layers.m;
+  const V one = P::splat(1.f), half = P::splat(.5f), mone = P::splat(-1.f);
+  const int last = m.L - 1;
+  V e[2];
+  {
+    const V wv = P::splat(w), iv = P::splat(m.ivs(last));
+    const V X = P::mul(P::fma(wv, iv, k), P::abs(P::fma(wv, P::splat(-m.ivs(last)), k)));
+    e[0] = P::mul(P::mul(X, P::rsqrt0(X)), P::splat(m.rho(last)));
+    e[1] = P::mul(iv, iv);
+  }
+  int ex[P::NL] = {};
+  V ev = P::splat(0.f);
+#pragma unroll 2
+  for (int l = last - 1; l >= m.water; --l) {
+    const LoveLayer32<P> ly = layers.get(l, w);
+    const V X = P::mul(P::add(k, ly.kj), P::abs(P::fma(ly.kj, mone, k)));
+    const V ir = P::rsqrt0(X), r = P::mul(X, ir), q = P::mul(r, ly.h);
+    V sn, cn;
+    sincos32<P>(q, &sn, &cn);
+    const V d = P::ex2(P::mul(q, P::splat(-1.4426950408889634f)));
+    const typename P::M prop = P::ltv(k, ly.kj);
+    const V c = P::sel(prop, cn, P::mul(half, P::fma(d, d, one)));
+    const V s = P::sel(prop, sn, P::mul(half, P::fma(P::mul(d, mone), d, one)));
+    const V y = P::sel(P::gt0(ir), P::mul(s, ir), ly.h);  // sin(r h) / r -> h as r -> 0
+    const V t = P::mul(r, s), z = P::sel(prop, P::neg(t), t);
+    ev = P::add(ev, P::sel(prop, P::splat(0.f), q));
+    const V u = P::fma(e[0], c, P::mul(P::mul(e[1], z), ly.mu));
+    e[1] = P::fma(e[1], c, P::mul(P::mul(e[0], y), ly.imu));
+    e[0] = u;
+    scale32<P>(e, ex);
+  }
+  const V n2 = P::add(P::fma(e[0], e[0], P::mul(e[1], e[1])), P::splat(1e-30f));
+#pragma unroll
+  for (int i = 0; i < P::NL; ++i) {
+    const float nn = lane_of(n2, i);
+    if (shape) lane_of(*shape, i) = x_mul(lane_of(e[0], i), rsqrtf(nn));
+    if (lmag)
+      lane_of(*lmag, i) =
+          x_fma(.5f, log2f(nn), x_fma(lane_of(ev, i), 1.4426950408889634f, static_cast<float>(ex[i])));
+  }
+  *F = e[0];
+}
+#endif
+
 // Love secular values (SH propagator) and shape features of S samples.
 template <class N, class T, int S>
 MD200_FN void love_multi(const LayerView<T> &m, const N *k, const N &w, N *F, N *shape,
                          typename Base<N>::type *lmag, typename Base<N>::type *levan = nullptr) {
   using B = typename Base<N>::type;
+#if defined(__CUDA_ARCH__)
+  // the scan's single-precision evaluations: explicitly rounded (love_eval32)
+  if constexpr (std::is_same<N, float>::value && std::is_same<T, float>::value && S == 1) {
+    if (levan == nullptr) {
+      love_eval32<R1>(Love1{m}, k[0], w, F, shape, lmag);
+      return;
+    }
+  }
+#endif
   const B tiny = sizeof(B) == 4 ? B(1e-30) : B(1e-40);
   const int last = m.L - 1;
   N e[S][2];

@@ -58,6 +58,9 @@ namespace md200 {
 #ifndef MD200_SPLIT_PAIR_BLOCKS
 #define MD200_SPLIT_PAIR_BLOCKS 4
 #endif
+#ifndef MD200_SPLIT_PAIR_BLOCKS_LOVE
+#define MD200_SPLIT_PAIR_BLOCKS_LOVE 6
+#endif
 #ifndef MD200_SPLIT_PAIR_GRID
 #define MD200_SPLIT_PAIR_GRID 64
 #endif
@@ -264,10 +267,10 @@ __global__ void __launch_bounds__(128, MD200_SPLIT_EVAL_BLOCKS) split_eval32(Dev
 }
 
 #if MD200_SPLIT_PAIR
-// Rayleigh: one thread per pair of sample slots of an active trace -- slot j of
-// its first 32-sample step and slot j of its second -- whose FP32 values come
-// from one paired evaluation (rayleigh_eval32<R2>: each half bit for bit the
-// single evaluation split_eval32 and the fused scan make).  A slot past the
+// One thread per pair of sample slots of an active trace -- slot j of its first
+// 32-sample step and slot j of its second -- whose FP32 values come from one paired
+// evaluation (rayleigh_eval32<R2>, love_eval32<R2>: each half bit for bit the
+// single evaluation the fused scan makes).  A slot past the
 // window or in the near-cutoff band leaves its half to a copy of the other
 // sample, whose result is not stored.
 static_assert(SPLIT_SAMPLES == 64, "the paired evaluation takes the two 32-sample steps of a round");
@@ -281,15 +284,17 @@ static_assert(SPLIT_SAMPLES == 64, "the paired evaluation takes the two 32-sampl
 // fewer instructions, FMA pipe 67 % busy; the FMA pipe's own time is 15 ms).
 // Dynamic shared memory: `buffers` (2, or 1 where two would cost resident CTAs)
 // x Ls records for each of the 4 warps.
-inline size_t split_pair_smem(int Ls, int buffers) {
-  return static_cast<size_t>(4) * buffers * Ls * PAIR_ROW * 2 * sizeof(float);
+inline size_t split_pair_smem(int wave, int Ls, int buffers) {
+  return static_cast<size_t>(4) * buffers * Ls * pair_row(wave) * 2 * sizeof(float);
 }
-inline int split_pair_buffers(int Ls) { return Ls <= 56 ? 2 : 1; }
+inline int split_pair_buffers(int wave, int Ls) { return Ls <= (wave ? 168 : 56) ? 2 : 1; }
 
-__global__ void __launch_bounds__(128, MD200_SPLIT_PAIR_BLOCKS) split_eval32_pair(Dev d, int p, int buffers) {
+template <int WAVE>
+__global__ void __launch_bounds__(128, WAVE ? MD200_SPLIT_PAIR_BLOCKS_LOVE : MD200_SPLIT_PAIR_BLOCKS)
+    split_eval32_pair(Dev d, int p, int buffers) {
   extern __shared__ __align__(16) float4 pair_rec[];
   const int lane = threadIdx.x & 31;
-  const int n16 = d.Ls * (PAIR_ROW / 2);  // 16-byte pieces of a model's records
+  const int n16 = d.Ls * (pair_row(WAVE) / 2);  // 16-byte pieces of a model's records
   float4 *mine = pair_rec + (threadIdx.x >> 5) * buffers * n16;
   const long long n = static_cast<long long>(d.ctr[C_SP_ACT0 + p]) * 32;
   const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
@@ -331,7 +336,8 @@ __global__ void __launch_bounds__(128, MD200_SPLIT_PAIR_BLOCKS) split_eval32_pai
         const float x0 = static_cast<float>(e0 ? c0 : c1), x1 = static_cast<float>(e1 ? c1 : c0);
         const float2 kk = make_float2(w / x0, w / x1);
         float2 F, g, M;
-        rayleigh_eval32<R2>(Layers2{view, mine + buf * n16}, kk, make_float2(w / kk.x, w / kk.y), w, &F, &g, &M);
+        if constexpr (WAVE) love_eval32<R2>(Love2{view, mine + buf * n16}, kk, w, &F, &g, &M);
+        else rayleigh_eval32<R2>(Layers2{view, mine + buf * n16}, kk, make_float2(w / kk.x, w / kk.y), w, &F, &g, &M);
         const unsigned long long ls = layer_steps(tr.L, tr.water);
         if (e0) {
           s0.F = F.x;
@@ -411,6 +417,11 @@ __device__ __forceinline__ bool needs_last_cell(const ScanState &st, int K) {
   return u > v + noise && v / ((u - v) / h0) < 1.25f * h0;
 }
 
+// Records a bookkeeping thread has on their way to shared memory: the loop is a
+// chain of dependent decisions, its loads need not be.  (One ahead, in registers,
+// it waited 8 warps an issue for memory.)
+constexpr int BOOK_AHEAD = 4;
+
 // One thread per active trace: its samples of this round in order, through the
 // bookkeeping of scan_bookkeep (one lane's share of it, carried sample by
 // sample).  Ends at the trace's K-th bracket, at the end of its window, at a
@@ -419,10 +430,20 @@ __device__ __forceinline__ bool needs_last_cell(const ScanState &st, int K) {
 template <int WAVE>
 __global__ void __launch_bounds__(128) split_book(Dev d, int p) {
   constexpr bool single = true;
+  __shared__ float4 ring[2][BOOK_AHEAD][128];
   const int lane = threadIdx.x & 31;
   const int n = d.ctr[C_SP_ACT0 + p];
   const int stride = gridDim.x * blockDim.x;
   const int n_pad = (n + 31) & ~31;
+  // record j of a trace's samples into this thread's ring
+  auto fetch = [&](const SplitSample *rec, int j) {
+    if (j < SPLIT_SAMPLES) {
+      const float4 *src = reinterpret_cast<const float4 *>(rec + j);
+      cp_async16(&ring[0][j % BOOK_AHEAD][threadIdx.x], src);
+      cp_async16(&ring[1][j % BOOK_AHEAD][threadIdx.x], src + 1);
+    }
+    asm volatile("cp.async.commit_group;\n" ::);
+  };
   // counters of the samples the bookkeeping consumes, as the fused scan counts
   // its steps' samples: each an FP32 evaluation, the re-evaluated ones also FP64
   unsigned long long ev = 0, ev32 = 0, sts = 0, sts32 = 0;
@@ -442,12 +463,19 @@ __global__ void __launch_bounds__(128) split_book(Dev d, int p) {
       const SplitTrace tr = d.sp_tr[i];
       const unsigned long long nsteps = layer_steps(tr.L, tr.water);
       bool stop = false;  // the K-th bracket, the window end or a non-finite value
-      // the next record is loaded while this one is worked on (the loop is a
-      // chain of dependent decisions; its loads need not be)
-      SplitSample ahead = d.sp_s[base];
+      for (int j = 0; j < BOOK_AHEAD; ++j) fetch(d.sp_s + base, j);
       for (int j = 0; j < SPLIT_SAMPLES; ++j) {
-        const SplitSample smp = ahead;
-        if (j + 1 < SPLIT_SAMPLES) ahead = d.sp_s[base + j + 1];
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(BOOK_AHEAD - 1) : "memory");
+        SplitSample smp;
+        {
+          const float4 a = ring[0][j % BOOK_AHEAD][threadIdx.x], b = ring[1][j % BOOK_AHEAD][threadIdx.x];
+          smp.c = __hiloint2double(__float_as_int(a.y), __float_as_int(a.x));
+          smp.F = __hiloint2double(__float_as_int(a.w), __float_as_int(a.z));
+          smp.g = b.x;
+          smp.M = b.y;
+          smp.k = __float_as_uint(b.z);
+        }
+        fetch(d.sp_s + base, j + BOOK_AHEAD);
         const double c = smp.c;
         if (!(c < INFINITY)) {  // the window is exhausted
           st.bits |= SS_FINISHED;
@@ -550,6 +578,7 @@ __global__ void __launch_bounds__(128) split_book(Dev d, int p) {
         go_on = true;  // the round's samples are used up: more next round
       }
       d.sp_state[t] = st;
+      asm volatile("cp.async.wait_all;\n" ::: "memory");  // (the next trace's records take the same places)
     }
     split_publish(d, t, st, publish, lane);
     const int za = warp_append(&d.ctr[C_SP_ZOOM], zoom ? 1 : 0, lane);
@@ -560,11 +589,13 @@ __global__ void __launch_bounds__(128) split_book(Dev d, int p) {
   split_count(d, ev, ev32, sts, sts32, lane);
 }
 
+// (Four resident CTAs: unbounded, 167 registers left room for three and a seventh of
+// the warps; the scan stage of 20,000 models 37.9 -> 37.1 ms.)
 // One warp per window request: a trough window (screened in FP32, zoomed in
 // FP64 unless dismissed) after which the trace goes on, or the last cell of a
 // finished trace, after which it is published.
 template <int WAVE>
-__global__ void __launch_bounds__(128) split_zoom(Dev d, int p) {
+__global__ void __launch_bounds__(128, 4) split_zoom(Dev d, int p) {
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const int n = d.ctr[C_SP_ZOOM];
   for (int r = blockIdx.x * (blockDim.x >> 5) + wib; r < n; r += gridDim.x * (blockDim.x >> 5)) {
