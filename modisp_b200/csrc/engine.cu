@@ -375,12 +375,15 @@ struct Ragged {
 constexpr int MODEL_LIST_MIN_TRACES = 4096;
 
 // Rounds of the split FP32 scan for a run of nt traces over an active set of
-// cap traces: enough for every trace of a typical run to finish (a trace takes
-// a round per SPLIT_SAMPLES samples, most take two or three); traces still
-// unfinished after them are handed to the fused kernel.
-int split_rounds(int nt, int cap) {
+// cap traces: enough for most traces to finish (a trace takes a round per
+// SPLIT_SAMPLES samples and one per trough window, most take three); those still
+// unfinished after them are handed to the fused kernel.  A round of nothing costs
+// 35-40 us of launches, a handed-over trace a warp's scan of its rest.  Measured best
+// at 3, 120 and 1,200 thousand traces: 3 (Love) and 4 rounds (Rayleigh) per
+// active set; with nine, 120,000 Rayleigh traces took 4.41 ms against 4.16.
+int split_rounds(int nt, int cap, int wave) {
   const int waves = (nt + cap - 1) / cap;
-  return std::min(md200_engine::MAX_SPLIT_ROUNDS, 3 * waves + 6);
+  return std::min(md200_engine::MAX_SPLIT_ROUNDS, 3 * waves + (wave == 0 ? 1 : 0));
 }
 
 // The split FP32 scan's launches (split_scan.cuh): `rounds` rounds, then the
@@ -393,8 +396,11 @@ int split_scan(md200_engine *e, const Dev &d, int rounds, cudaStream_t s) {
   const int cap = d.sp_cap;
   const int fill_blocks = std::max(1, std::min((cap + 255) / 256, sms * 8));
   const int pos_blocks = std::max(1, std::min((cap + 3) / 4, sms * 16));
+  const int eval_blocks = std::max(1, std::min((cap + 3) / 4, sms * MD200_SPLIT_PAIR_GRID));
   const int buffers = split_pair_buffers(WAVE, d.Ls);
   const int book_blocks = std::max(1, std::min((cap + 127) / 128, sms * 8));
+  const int redo_blocks = std::max(1, std::min((cap + 3) / 4, sms * 8));
+  const int zoom_blocks = std::max(1, std::min((cap + 15) / 16, sms * 8));
   int nl = 0;
   for (int r = 0; r < rounds; ++r) {
     const int p = r & 1;
@@ -404,14 +410,14 @@ int split_scan(md200_engine *e, const Dev &d, int rounds, cudaStream_t s) {
     if (!e->capturing && cudaEventRecord(e->sp_ev[2 * r], s) != cudaSuccess) return -1;
 #if MD200_SPLIT_PAIR
     split_eval32_pair<WAVE>
-        <<<sms * MD200_SPLIT_PAIR_GRID, 128, split_pair_smem(WAVE, d.Ls, buffers), s>>>(d, p, buffers);
+        <<<eval_blocks, 128, split_pair_smem(WAVE, d.Ls, buffers), s>>>(d, p, buffers);
 #else
     split_eval32<WAVE><<<sms * 16, 128, 0, s>>>(d, p);
 #endif
     if (!e->capturing && cudaEventRecord(e->sp_ev[2 * r + 1], s) != cudaSuccess) return -1;
-    split_redo<WAVE><<<sms * 8, 128, 0, s>>>(d, p);
+    split_redo<WAVE><<<redo_blocks, 128, 0, s>>>(d, p);
     split_book<WAVE><<<book_blocks, 128, 0, s>>>(d, p);
-    split_zoom<WAVE><<<sms * 8, 128, 0, s>>>(d, p);
+    split_zoom<WAVE><<<zoom_blocks, 128, 0, s>>>(d, p);
     nl += 7;
   }
   e->sp_timed = e->capturing ? 0 : rounds;
@@ -491,18 +497,17 @@ int enqueue(md200_engine *e, const double *h, const double *vp, const double *vs
     MD200_CK(cudaGetLastError());
   }
   MD200_CK(mark(2));
-  // the split scan in auto mode: Rayleigh runs of SPLIT_MIN_TRACES traces or more
-  // (the Love step is too cheap for the rounds to pay: measured slower)
   // larger runs list their brackets and roots model by model (below a few thousand
   // traces refinement is latency-bound and the extra launches cost what it gains)
   Dev dm = d;
   dm.model_lists = nt >= MODEL_LIST_MIN_TRACES ? 1 : 0;
   const int model_blocks = (B + 3) / 4;
   const auto refine_fn = wave == 0 ? refine<0> : refine<1>;
+  // the split scan in auto mode: where its rounds beat the fused kernel
   const bool split = d.fp32 && (e->o.scan_mode == 2 ||
-                                (e->o.scan_mode == 0 && wave == 0 && nt >= SPLIT_MIN_TRACES));
+                                (e->o.scan_mode == 0 && nt >= SPLIT_MIN_TRACES[wave]));
   if (split) {
-    const int rounds = split_rounds(nt, d.sp_cap);
+    const int rounds = split_rounds(nt, d.sp_cap, wave);
     const int launched = wave == 0 ? split_scan<0>(e, dm, rounds, s) : split_scan<1>(e, dm, rounds, s);
     if (launched < 0) return fail("modisp_b200 CUDA: event record failed in the split scan");
     nl += launched;

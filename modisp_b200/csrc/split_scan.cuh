@@ -67,7 +67,11 @@ namespace md200 {
 constexpr int SPLIT_STEPS = MD200_SPLIT_STEPS;    // 32-sample steps per trace per round
 constexpr int SPLIT_SAMPLES = 32 * SPLIT_STEPS;  // sample slots per active trace
 constexpr int SPLIT_ACTIVE_MAX = 1 << 20;         // active-set capacity (traces)
-constexpr int SPLIT_MIN_TRACES = 4096;            // runs with fewer traces use the fused kernel
+// Runs with fewer traces use the fused kernel.  Scan stage, fused against split:
+// Rayleigh 9,000 traces 0.58 / 0.75 ms, 30,000 1.68 / 1.36, 120,000 6.65 / 4.16,
+// 1.2 million 78 / 37; Love, whose step is a tenth of the work, 30,000 0.50 / 0.65,
+// 120,000 1.91 / 1.97, 1.2 million 19.2 / 17.2.
+constexpr int SPLIT_MIN_TRACES[2] = {16384, 131072};
 constexpr unsigned SK_SEED = 1, SK_NEAR = 2, SK_EXACT = 4, SK_REDO = 8;
 constexpr int ZOOM_TROUGH = 0, ZOOM_LAST = 1;
 
