@@ -460,7 +460,7 @@ MD200_HD bool root_adjoint(const LayerView<double> &m, const double *tab, double
 // Adjoint mode: grad [4][B][Lmax] += wc[cell] dc/dm + wu[cell] dU/dm.
 // ---------------------------------------------------------------------------
 template <int WAVE>
-__global__ void __launch_bounds__(128) root_jacobians(Dev d, const double *vel, const double *grp, double *jac_c,
+__global__ void __launch_bounds__(WAVE ? 128 : 256) root_jacobians(Dev d, const double *vel, const double *grp, double *jac_c,
                                                       double *jac_u, const double *wc, const double *wu,
                                                       double *grad, int *nfail) {
   const int nm = d.nmodes, T = d.T, Lmax = d.Lmax;

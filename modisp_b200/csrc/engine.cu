@@ -693,17 +693,27 @@ int jacobian_enqueue(md200_engine *e, const double *h, const double *vp, const d
   d.pred = nullptr;
   MD200_CK(cudaMemsetAsync(d.ctr, 0, sizeof(int) * C_COUNT, s));
   const int pw = e->prep_warps;
-  prep_models<<<(B + pw - 1) / pw, 32 * pw, e->prep_smem, s>>>(d, e->sortcap, 0);
+  prep_models<<<(B + pw - 1) / pw, 32 * pw, e->prep_smem, s>>>(d, e->sortcap, 1);
   MD200_CK(cudaGetLastError());
   if (grad) MD200_CK(cudaMemsetAsync(grad, 0, sizeof(double) * 4 * static_cast<size_t>(B) * e->L, s));
   // One thread per output cell.  Most cells hold no root and their warps leave at
   // once; the block scheduler then keeps every SM on root-bearing warps.  A grid
   // capped at the resident blocks (each thread striding over many cells) left
   // threads with uneven shares and ran 3.2x slower.
+  //
+  // Eight warps fit an SM (255 registers), and a Rayleigh layer's forward and adjoint
+  // steps are longer than the instruction cache: warps of one block, which start
+  // together, fetch them together.  One block of 256 an SM instead of two of 128, full
+  // Jacobians of 12-layer models: 4,096 models 7.15 -> 5.99 ms, 1,024 1.68 -> 1.61; with
+  // less than two blocks an SM the rest of a block idles (64 models: 0.36 ms with 256
+  // threads, 0.28 with 128, 0.24 with 64).  Love's short steps fit: 128 throughout
+  // (1,024 models 0.32 ms, 0.37 with 256).
   const long long cells = static_cast<long long>(B) * e->nmodes * e->T;
-  const int blocks = static_cast<int>(std::min<long long>((cells + 127) / 128, 1LL << 30));
-  if (wave == 0) root_jacobians<0><<<blocks, 128, 0, s>>>(d, vel, grp, jc, ju, wc, wu, grad, d.ctr + C_JFAIL);
-  else root_jacobians<1><<<blocks, 128, 0, s>>>(d, vel, grp, jc, ju, wc, wu, grad, d.ctr + C_JFAIL);
+  const int sms = e->list_blocks / 8;
+  const int threads = wave == 0 && cells >= 512LL * sms ? 256 : wave == 0 && cells <= 128LL * sms ? 64 : 128;
+  const int blocks = static_cast<int>(std::min<long long>((cells + threads - 1) / threads, 1LL << 30));
+  if (wave == 0) root_jacobians<0><<<blocks, threads, 0, s>>>(d, vel, grp, jc, ju, wc, wu, grad, d.ctr + C_JFAIL);
+  else root_jacobians<1><<<blocks, threads, 0, s>>>(d, vel, grp, jc, ju, wc, wu, grad, d.ctr + C_JFAIL);
   MD200_CK(cudaGetLastError());
   return 0;
 }

@@ -226,7 +226,9 @@ constexpr int SCAN_START_MARGIN = 6;
 // prep_models: one warp per model.
 // Shared memory per warp: 2 * sortcap doubles + 2 * sortcap ints.
 // ---------------------------------------------------------------------------
-__global__ void prep_models(Dev d, int sortcap, int automatic) {
+// With `tables`, only what the Jacobian kernel reads: the layer tables and the
+// model's state (its window is automatic, so never empty).
+__global__ void prep_models(Dev d, int sortcap, int tables) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const int b = blockIdx.x * (blockDim.x >> 5) + wib;
@@ -265,7 +267,7 @@ __global__ void prep_models(Dev d, int sortcap, int automatic) {
         t64[q * Ls + r] = vals[q];
         t32[q * Ls + r] = static_cast<float>(vals[q]);
       }
-      if (d.fp32) {  // the paired evaluation's record of this layer
+      if (d.fp32 && !tables) {  // the paired evaluation's record of this layer
         const float h = static_cast<float>(vals[0]), vs2 = static_cast<float>(vals[3]), rho = static_cast<float>(vals[4]);
         const float irho = static_cast<float>(vals[5]), nrho2 = -x_mul(rho, rho), nirho2 = -x_mul(irho, irho);
         const float rec[PAIR_ROW] = {h,    static_cast<float>(vals[1]), static_cast<float>(vals[2]),
@@ -294,7 +296,7 @@ __global__ void prep_models(Dev d, int sortcap, int automatic) {
   //    shear velocity (exclusive).
   double lo = d.bounds_in ? d.bounds_in[2 * b] : 0.;
   double hi = d.bounds_in ? d.bounds_in[2 * b + 1] : INFINITY;
-  if (automatic || !(lo > 0.)) {
+  if (!tables && !(lo > 0.)) {
     double best = 1e300;
     for (int j = top + lane; j < L; j += 32) {
       if (hr[j] == 0. && j < L - 1) continue;  // a zero-thickness row carries no waves
@@ -326,7 +328,7 @@ __global__ void prep_models(Dev d, int sortcap, int automatic) {
       d.bounds_out[2 * b + 1] = hi;
     }
   }
-  if (state) return;
+  if (state || tables) return;
 
   // 3. knot table: log-spaced points over [lo, hi] plus every finite-layer body
   //    velocity inside the window (kinks of N(c)), sorted.

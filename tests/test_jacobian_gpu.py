@@ -222,3 +222,30 @@ def test_jacobians_at_the_largest_layer_count(wave, single, oracle_lib):
         worst = max(worst, _row_err(jc[b, m, f], oracle_lib.phase_jacobian(*row, periods[f], v[b, m, f], wave)))
         assert np.isfinite(ju[b, m, f]).all()
     assert worst < PHASE_TOL_ORACLE, worst
+
+
+@pytest.mark.parametrize("wave", ["rayleigh", "love"])
+def test_jacobians_do_not_depend_on_the_batch(wave):
+    """Large, middle and small batches take blocks of different sizes: the same Jacobians bit for bit,
+    rows of zero thickness and models without a guide included."""
+    import torch
+    from modisp_b200 import workloads
+    from modisp_b200.autograd import DifferentiableSolver
+    B, T, nm = 650, 40, 3
+    b = workloads.crustal_batch(B, 9, nmin=1, nmax=6)
+    b["vs"][::11], b["vp"][::11] = 1.5, 2.9  # no layer slower than the half-space
+    x = [torch.from_numpy(b[k]).cuda() for k in ("thickness", "vp", "vs", "rho")]
+    periods = np.geomspace(.5, 20., T)
+
+    def solve(lo, hi):
+        s = DifferentiableSolver(hi - lo, x[0].shape[1], periods, nm, wave=wave)
+        out = s.jacobian(*[v[lo:hi] for v in x])
+        s.close()
+        return out
+
+    whole = solve(0, B)
+    for size in (200, 90):  # more and fewer cells than 128 an SM
+        for lo in range(0, B, size):
+            hi = min(B, lo + size)
+            for w, p in zip(whole, solve(lo, hi)):
+                assert torch.equal(torch.nan_to_num(w[lo:hi], nan=-7.), torch.nan_to_num(p, nan=-7.))
