@@ -110,7 +110,7 @@ struct md200_engine {
   md200_options o{};
   cudaStream_t stream = nullptr;
   Dev d{};
-  int sortcap = 0, prep_warps = 4, scan_warps = 4, scan_blocks64 = 0, scan_blocks32 = 0;
+  int sortcap = 0, bodycap = 0, prep_warps = 4, scan_warps = 4, scan_blocks64 = 0, scan_blocks32 = 0;
   int list_blocks = 0;
   size_t scan_smem64 = 0, scan_smem32 = 0, prep_smem = 0;
   // host-path buffers
@@ -337,7 +337,10 @@ int setup(md200_engine *e, bool staging) {
   while (cap2 < sort_n) cap2 <<= 1;
   e->sortcap = cap2;
   e->prep_warps = 4;
-  e->prep_smem = static_cast<size_t>(e->prep_warps) * cap2 * (sizeof(double) + sizeof(int));
+  int body2 = 1;
+  while (body2 < 2 * L) body2 <<= 1;
+  e->bodycap = body2;
+  e->prep_smem = static_cast<size_t>(e->prep_warps) * (cap2 * (sizeof(double) + sizeof(int)) + body2 * sizeof(double));
   for (auto &x : e->ev) MD200_CK(cudaEventCreate(&x));
   for (auto &x : e->chunk_ev) MD200_CK(cudaEventCreateWithFlags(&x, cudaEventDisableTiming));
   for (auto &x : e->solved_ev) MD200_CK(cudaEventCreateWithFlags(&x, cudaEventDisableTiming));
@@ -479,7 +482,7 @@ int enqueue(md200_engine *e, const double *h, const double *vp, const double *vs
   auto mark = [&](int i) { return e->capturing ? cudaSuccess : cudaEventRecord(e->ev[i], s); };
   MD200_CK(mark(0));
   const int pw = e->prep_warps;
-  prep_models<<<(B + pw - 1) / pw, 32 * pw, e->prep_smem, s>>>(d, e->sortcap, 0);
+  prep_models<<<(B + pw - 1) / pw, 32 * pw, e->prep_smem, s>>>(d, e->sortcap, e->bodycap, 0);
   ++nl;
   MD200_CK(cudaGetLastError());
   if (cont) {
@@ -503,6 +506,15 @@ int enqueue(md200_engine *e, const double *h, const double *vp, const double *vs
   dm.model_lists = nt >= MODEL_LIST_MIN_TRACES ? 1 : 0;
   const int model_blocks = (B + 3) / 4;
   const auto refine_fn = wave == 0 ? refine<0> : refine<1>;
+  // grids no larger than the run can fill: blocks with nothing to do cost a small
+  // run more than its work (an empty pass of four kernels at full grids 27 us)
+  auto within = [](int blocks, long long items, int per_block) {
+    return static_cast<unsigned>(std::max<long long>(1, std::min<long long>(blocks, (items + per_block - 1) / per_block)));
+  };
+  const unsigned refine_blocks = within(e->list_blocks, static_cast<long long>(nt) * d.KB, 128);
+  const unsigned group_blocks = within(e->list_blocks, static_cast<long long>(nt) * d.nmodes, 128);
+  const unsigned scan64_blocks = within(e->scan_blocks64, nt, e->scan_warps);
+  const unsigned scan_blocks = within(d.fp32 ? e->scan_blocks32 : e->scan_blocks64, nt, e->scan_warps);
   // the split scan in auto mode: where its rounds beat the fused kernel
   const bool split = d.fp32 && (e->o.scan_mode == 2 ||
                                 (e->o.scan_mode == 0 && nt >= SPLIT_MIN_TRACES[wave]));
@@ -513,7 +525,7 @@ int enqueue(md200_engine *e, const double *h, const double *vp, const double *vs
     nl += launched;
   } else {
     e->sp_timed = 0;
-    const dim3 grid(d.fp32 ? e->scan_blocks32 : e->scan_blocks64), block(32 * e->scan_warps);
+    const dim3 grid(scan_blocks), block(32 * e->scan_warps);
     const size_t sm = d.fp32 ? e->scan_smem32 : e->scan_smem64;
     if (d.fp32 && wave == 0) scan<float, 0><<<grid, block, sm, s>>>(dm, d.trace_list, C_SCAN_CURSOR, C_NTRACE);
     else if (d.fp32) scan<float, 1><<<grid, block, sm, s>>>(dm, d.trace_list, C_SCAN_CURSOR, C_NTRACE);
@@ -527,7 +539,7 @@ int enqueue(md200_engine *e, const double *h, const double *vp, const double *vs
     list_brackets<<<model_blocks, 128, 0, s>>>(d);
     ++nl;
   }
-  refine_fn<<<e->list_blocks, 128, 0, s>>>(d);
+  refine_fn<<<refine_blocks, 128, 0, s>>>(d);
   ++nl;
   MD200_CK(cudaGetLastError());
   MD200_CK(mark(4));
@@ -536,14 +548,14 @@ int enqueue(md200_engine *e, const double *h, const double *vp, const double *vs
     ++nl;
     MD200_CK(mark(5));
     if (wave == 0)
-      scan<double, 0><<<e->scan_blocks64, 32 * e->scan_warps, e->scan_smem64, s>>>(d, d.repair_list,
+      scan<double, 0><<<scan64_blocks, 32 * e->scan_warps, e->scan_smem64, s>>>(d, d.repair_list,
                                                                                  C_REPAIR_CURSOR, C_NREPAIR);
     else
-      scan<double, 1><<<e->scan_blocks64, 32 * e->scan_warps, e->scan_smem64, s>>>(d, d.repair_list,
+      scan<double, 1><<<scan64_blocks, 32 * e->scan_warps, e->scan_smem64, s>>>(d, d.repair_list,
                                                                                  C_REPAIR_CURSOR, C_NREPAIR);
     ++nl;
     MD200_CK(mark(6));
-    refine_fn<<<e->list_blocks, 128, 0, s>>>(d);
+    refine_fn<<<refine_blocks, 128, 0, s>>>(d);
     ++nl;
     MD200_CK(cudaGetLastError());
   } else {
@@ -560,7 +572,7 @@ int enqueue(md200_engine *e, const double *h, const double *vp, const double *vs
       list_roots<<<model_blocks, 128, 0, s>>>(d);
       ++nl;
     }
-    group_velocity<<<e->list_blocks, 128, 0, s>>>(d);
+    group_velocity<<<group_blocks, 128, 0, s>>>(d);
     ++nl;
     MD200_CK(cudaGetLastError());
   }
@@ -574,20 +586,20 @@ int enqueue(md200_engine *e, const double *h, const double *vp, const double *vs
     Dev df = d;
     df.jmax = JMAX_FALLBACK;
     if (wave == 0)
-      scan<double, 0><<<e->scan_blocks64, 32 * e->scan_warps, e->scan_smem64, s>>>(df, d.repair_list,
+      scan<double, 0><<<scan64_blocks, 32 * e->scan_warps, e->scan_smem64, s>>>(df, d.repair_list,
                                                                                  C_REPAIR_CURSOR, C_NREPAIR);
     else
-      scan<double, 1><<<e->scan_blocks64, 32 * e->scan_warps, e->scan_smem64, s>>>(df, d.repair_list,
+      scan<double, 1><<<scan64_blocks, 32 * e->scan_warps, e->scan_smem64, s>>>(df, d.repair_list,
                                                                                  C_REPAIR_CURSOR, C_NREPAIR);
     ++nl;
     MD200_CK(cudaGetLastError());
-    refine_fn<<<e->list_blocks, 128, 0, s>>>(d);
+    refine_fn<<<refine_blocks, 128, 0, s>>>(d);
     ++nl;
     assemble<<<(nt + 255) / 256, 256, 0, s>>>(d, d.repair_list, C_NREPAIR);
     ++nl;
     MD200_CK(cudaGetLastError());
     if (d.group) {
-      group_velocity<<<e->list_blocks, 128, 0, s>>>(d);
+      group_velocity<<<group_blocks, 128, 0, s>>>(d);
       ++nl;
       MD200_CK(cudaGetLastError());
     }
@@ -607,19 +619,19 @@ int enqueue(md200_engine *e, const double *h, const double *vp, const double *vs
     ++nl;
     MD200_CK(cudaGetLastError());
     if (wave == 0)
-      scan<double, 0><<<e->scan_blocks64, 32 * e->scan_warps, e->scan_smem64, s>>>(d, d.repair_list,
+      scan<double, 0><<<scan64_blocks, 32 * e->scan_warps, e->scan_smem64, s>>>(d, d.repair_list,
                                                                                  C_REPAIR_CURSOR, C_NREPAIR);
     else
-      scan<double, 1><<<e->scan_blocks64, 32 * e->scan_warps, e->scan_smem64, s>>>(d, d.repair_list,
+      scan<double, 1><<<scan64_blocks, 32 * e->scan_warps, e->scan_smem64, s>>>(d, d.repair_list,
                                                                                  C_REPAIR_CURSOR, C_NREPAIR);
     ++nl;
-    refine_fn<<<e->list_blocks, 128, 0, s>>>(d);
+    refine_fn<<<refine_blocks, 128, 0, s>>>(d);
     ++nl;
     assemble<<<(nt + 255) / 256, 256, 0, s>>>(d, d.cont_list, C_NTARGET);
     ++nl;
     MD200_CK(cudaGetLastError());
     if (d.group) {
-      group_velocity<<<e->list_blocks, 128, 0, s>>>(d);
+      group_velocity<<<group_blocks, 128, 0, s>>>(d);
       ++nl;
       MD200_CK(cudaGetLastError());
     }
@@ -633,20 +645,20 @@ int enqueue(md200_engine *e, const double *h, const double *vp, const double *vs
     ++nl;
     MD200_CK(cudaGetLastError());
     if (wave == 0)
-      scan<double, 0><<<e->scan_blocks64, 32 * e->scan_warps, e->scan_smem64, s>>>(d, d.repair_list,
+      scan<double, 0><<<scan64_blocks, 32 * e->scan_warps, e->scan_smem64, s>>>(d, d.repair_list,
                                                                                  C_REPAIR_CURSOR, C_NREPAIR);
     else
-      scan<double, 1><<<e->scan_blocks64, 32 * e->scan_warps, e->scan_smem64, s>>>(d, d.repair_list,
+      scan<double, 1><<<scan64_blocks, 32 * e->scan_warps, e->scan_smem64, s>>>(d, d.repair_list,
                                                                                  C_REPAIR_CURSOR, C_NREPAIR);
     ++nl;
     MD200_CK(cudaGetLastError());
-    refine_fn<<<e->list_blocks, 128, 0, s>>>(d);
+    refine_fn<<<refine_blocks, 128, 0, s>>>(d);
     ++nl;
     assemble<<<(nt + 255) / 256, 256, 0, s>>>(d, d.repair_list, C_NREPAIR);
     ++nl;
     MD200_CK(cudaGetLastError());
     if (d.group) {
-      group_velocity<<<e->list_blocks, 128, 0, s>>>(d);
+      group_velocity<<<group_blocks, 128, 0, s>>>(d);
       ++nl;
       MD200_CK(cudaGetLastError());
     }
@@ -693,7 +705,7 @@ int jacobian_enqueue(md200_engine *e, const double *h, const double *vp, const d
   d.pred = nullptr;
   MD200_CK(cudaMemsetAsync(d.ctr, 0, sizeof(int) * C_COUNT, s));
   const int pw = e->prep_warps;
-  prep_models<<<(B + pw - 1) / pw, 32 * pw, e->prep_smem, s>>>(d, e->sortcap, 1);
+  prep_models<<<(B + pw - 1) / pw, 32 * pw, e->prep_smem, s>>>(d, e->sortcap, e->bodycap, 1);
   MD200_CK(cudaGetLastError());
   if (grad) MD200_CK(cudaMemsetAsync(grad, 0, sizeof(double) * 4 * static_cast<size_t>(B) * e->L, s));
   // One thread per output cell.  Most cells hold no root and their warps leave at

@@ -102,7 +102,9 @@ __device__ __noinline__ double eval64_outline(const LayerView<double> &m, int wa
 // Rayleigh cubic (cpp/common/physics.hpp:140-144).  Every operation is rounded
 // separately (no FMA contraction), matching the reference's -ffp-contract=off
 // build bit for bit: the search window is reported and compared exactly.
-__device__ double rayleigh_speed(double vp, double vs) {
+// (The bisections are called, not inlined: a model's preparation runs each once or
+// twice, and for a single model the time is that of fetching its code.)
+__device__ __noinline__ double rayleigh_speed(double vp, double vs) {
   const double q = __ddiv_rn(vs, vp), ratio = __dmul_rn(q, q);
   double l = 0., h = 1.;
   for (int j = 0; j < 56; ++j) {
@@ -117,7 +119,7 @@ __device__ double rayleigh_speed(double vp, double vs) {
 
 // Scholte-wave speed of a fluid over a solid half-space by bisection
 // (cpp/common/physics.hpp:146-156), separately rounded like rayleigh_speed.
-__device__ double scholte_speed(double vf, double rf, double vp, double vs, double rs) {
+__device__ __noinline__ double scholte_speed(double vf, double rf, double vp, double vs, double rs) {
   const double q1 = __ddiv_rn(vs, vp), ratio = __dmul_rn(q1, q1);
   const double q2 = __ddiv_rn(vs, vf), qf = __dmul_rn(q2, q2);
   double l = 0., h = fmax(0., __dmul_rn(fmin(1., __ddiv_rn(vf, vs)), __dadd_rn(1., -1e-12)));
@@ -135,8 +137,8 @@ __device__ double scholte_speed(double vf, double rf, double vp, double vs, doub
   return __dmul_rn(vs, __dmul_rn(__dadd_rn(l, h), .5));
 }
 
-// Warp-cooperative bitonic sort of n2 (a power of two) keys with int payloads.
-__device__ void warp_bitonic(double *key, int *val, int n2, int lane) {
+// Warp-cooperative bitonic sort of n2 (a power of two) keys.
+__device__ __noinline__ void warp_bitonic(double *key, int n2, int lane) {
   for (int size = 2; size <= n2; size <<= 1) {
     for (int stride = size >> 1; stride > 0; stride >>= 1) {
       for (int i = lane; i < (n2 >> 1); i += 32) {
@@ -147,9 +149,6 @@ __device__ void warp_bitonic(double *key, int *val, int n2, int lane) {
         if ((a > b) == up) {
           key[lo] = b;
           key[hi] = a;
-          const int t = val[lo];
-          val[lo] = val[hi];
-          val[hi] = t;
         }
       }
       __syncwarp();
@@ -224,19 +223,21 @@ constexpr int SCAN_START_MARGIN = 6;
 
 // ---------------------------------------------------------------------------
 // prep_models: one warp per model.
-// Shared memory per warp: 2 * sortcap doubles + 2 * sortcap ints.
+// Shared memory per warp: sortcap doubles and ints, bodycap doubles.
 // ---------------------------------------------------------------------------
 // With `tables`, only what the Jacobian kernel reads: the layer tables and the
 // model's state (its window is automatic, so never empty).
-__global__ void prep_models(Dev d, int sortcap, int tables) {
+__global__ void prep_models(Dev d, int sortcap, int bodycap, int tables) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const int b = blockIdx.x * (blockDim.x >> 5) + wib;
   if (b >= d.B) return;
   double *skey = reinterpret_cast<double *>(smem_raw) + static_cast<size_t>(wib) * sortcap;
   int *sval = reinterpret_cast<int *>(reinterpret_cast<double *>(smem_raw) +
-                                      static_cast<size_t>(blockDim.x >> 5) * sortcap) +
+                                      static_cast<size_t>(blockDim.x >> 5) * (sortcap + bodycap)) +
               static_cast<size_t>(wib) * sortcap;
+  double *bkey = reinterpret_cast<double *>(smem_raw) + static_cast<size_t>(blockDim.x >> 5) * sortcap +
+                 static_cast<size_t>(wib) * bodycap;
   const int Lmax = d.Lmax, Ls = d.Ls;
   const size_t in = static_cast<size_t>(b) * Lmax;
   double *t64 = d.layer64 + static_cast<size_t>(b) * ROWS * Ls;
@@ -296,12 +297,14 @@ __global__ void prep_models(Dev d, int sortcap, int tables) {
   //    shear velocity (exclusive).
   double lo = d.bounds_in ? d.bounds_in[2 * b] : 0.;
   double hi = d.bounds_in ? d.bounds_in[2 * b + 1] : INFINITY;
+  double top_speed = NAN;  // Rayleigh speed of the first solid row, where the window needed it
   if (!tables && !(lo > 0.)) {
     double best = 1e300;
     for (int j = top + lane; j < L; j += 32) {
       if (hr[j] == 0. && j < L - 1) continue;  // a zero-thickness row carries no waves
       const double s = vsr[j], p = vpr[j];
       double x = wave ? s : rayleigh_speed(p, s);
+      if (j == top) top_speed = x;
       if (!wave && top) x = fmin(x, scholte_speed(vpr[0], rr[0], p, s, rr[j]));
       best = fmin(best, x);
     }
@@ -332,14 +335,12 @@ __global__ void prep_models(Dev d, int sortcap, int tables) {
 
   // 3. knot table: log-spaced points over [lo, hi] plus every finite-layer body
   //    velocity inside the window (kinks of N(c)), sorted.
+  //    The log points are in order already: the body velocities are sorted on their
+  //    own, every log point takes its place after the body velocities below it, and
+  //    those fill the places left.
   const int nlog = d.nlog;
   const double lspan = log(hi / lo);
-  int n = 0;
-  for (int i = lane; i <= nlog; i += 32) {
-    skey[i] = i == 0 ? lo : (i == nlog ? hi : lo * exp(lspan * i / nlog));
-    sval[i] = 0;
-  }
-  n = nlog + 1;
+  int nb = 0;
   for (int base = top; base < L - 1; base += 32) {
     const int j = base + lane;
     bool ks = false, kp = false;
@@ -351,26 +352,37 @@ __global__ void prep_models(Dev d, int sortcap, int tables) {
       kp = !wave && p > lo && p < hi;
     }
     const unsigned ms = __ballot_sync(FULL, ks), mp = __ballot_sync(FULL, kp);
-    if (ks) {
-      const int r = n + __popc(ms & lanemask_lt());
-      skey[r] = s;
-      sval[r] = 1;
-    }
-    n += __popc(ms);
-    if (kp) {
-      const int r = n + __popc(mp & lanemask_lt());
-      skey[r] = p;
-      sval[r] = 1;
-    }
-    n += __popc(mp);
+    if (ks) bkey[nb + __popc(ms & lanemask_lt())] = s;
+    nb += __popc(ms);
+    if (kp) bkey[nb + __popc(mp & lanemask_lt())] = p;
+    nb += __popc(mp);
   }
-  int n2 = pow2_ceil(n);
-  for (int i = n + lane; i < n2; i += 32) {
-    skey[i] = INFINITY;
-    sval[i] = 0;
+  int n2 = pow2_ceil(nb);
+  for (int i = nb + lane; i < n2; i += 32) bkey[i] = INFINITY;
+  int n = nlog + 1 + nb;
+  for (int i = lane; i < n; i += 32) sval[i] = 1;
+  __syncwarp();
+  warp_bitonic(bkey, n2, lane);
+  for (int i = lane; i <= nlog; i += 32) {
+    const double v = i == 0 ? lo : (i == nlog ? hi : lo * exp(lspan * i / nlog));
+    int below = 0, end = nb;  // body velocities below v
+    while (below < end) {
+      const int mid = (below + end) >> 1;
+      if (bkey[mid] < v) below = mid + 1;
+      else end = mid;
+    }
+    skey[i + below] = v;
+    sval[i + below] = 0;
   }
   __syncwarp();
-  warp_bitonic(skey, sval, n2, lane);
+  for (int base = 0, j = 0; base < n; base += 32) {
+    const int i = base + lane;
+    const bool free = i < n && sval[i] == 1;
+    const unsigned m = __ballot_sync(FULL, free);
+    if (free) skey[i] = bkey[j + __popc(m & lanemask_lt())];
+    j += __popc(m);
+  }
+  __syncwarp();
   // Keep the last element of each run of equal keys, merging kink marks.
   int nk = 0;
   double4 *kt = d.knot + static_cast<size_t>(b) * d.nkmax;
@@ -440,15 +452,12 @@ __global__ void prep_models(Dev d, int sortcap, int tables) {
     }
     const int total = __shfl_sync(FULL, off, 31);
     off -= cnt;
-    for (int q = 0; q < cnt; ++q) {
-      skey[n + off + q] = v[q];
-      sval[n + off + q] = 0;
-    }
+    for (int q = 0; q < cnt; ++q) skey[n + off + q] = v[q];
     n += total;
   }
   __syncwarp();
   if (lane == 0) {
-    const double s0 = wave ? vsr[top] : rayleigh_speed(vpr[top], vsr[top]);
+    const double s0 = wave ? vsr[top] : isnan(top_speed) ? rayleigh_speed(vpr[top], vsr[top]) : top_speed;
     const double ws = (!wave && top) ? scholte_speed(vpr[0], rr[0], vpr[1], vsr[1], rr[1]) : NAN;
     const double gaps[5] = {1e-7, 1e-6, 1e-5, 1e-4, 1e-3};
     const double base[2] = {s0, ws};
@@ -470,9 +479,8 @@ __global__ void prep_models(Dev d, int sortcap, int tables) {
   __syncwarp();
   n2 = pow2_ceil(n);
   for (int i = n + lane; i < n2; i += 32) skey[i] = INFINITY;
-  for (int i = lane; i < n2; i += 32) sval[i] = 0;
   __syncwarp();
-  warp_bitonic(skey, sval, n2, lane);
+  warp_bitonic(skey, n2, lane);
   // 5. where the scan starts: a few grid points below the slowest velocity a root
   //    can have (lowest_root), on the same grid positions as a scan from the
   //    window's lower end.  Below every body velocity N(c) = 0, so grid point j
