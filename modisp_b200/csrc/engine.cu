@@ -285,7 +285,7 @@ int setup(md200_engine *e, bool staging) {
     d.sp_cap = static_cast<int>(std::min<size_t>(nt, SPLIT_ACTIVE_MAX));
     const size_t ns = static_cast<size_t>(d.sp_cap) * SPLIT_SAMPLES;
     if (plan_alloc(e, &d.sp_act[0], d.sp_cap) || plan_alloc(e, &d.sp_act[1], d.sp_cap) ||
-        plan_alloc(e, &d.sp_state, nt) || plan_alloc(e, &d.sp_s, ns) || plan_alloc(e, &d.sp_tr, d.sp_cap) ||
+        plan_alloc(e, &d.sp_state, nt) || plan_alloc(e, &d.sp_s, d.sp_cap) || plan_alloc(e, &d.sp_tr, d.sp_cap) ||
         plan_alloc(e, &d.sp_kf, nt) ||
         plan_alloc(e, &d.sp_redo, ns) || plan_alloc(e, &d.sp_zoom, d.sp_cap) ||
         plan_alloc(e, &d.sp_zarg, static_cast<size_t>(d.sp_cap) * 8))
@@ -411,12 +411,8 @@ int split_scan(md200_engine *e, const Dev &d, int rounds, cudaStream_t s) {
     split_feed_fill<<<fill_blocks, 256, 0, s>>>(d, p);
     split_positions<<<pos_blocks, 128, 0, s>>>(d, p);
     if (!e->capturing && cudaEventRecord(e->sp_ev[2 * r], s) != cudaSuccess) return -1;
-#if MD200_SPLIT_PAIR
     split_eval32_pair<WAVE>
         <<<eval_blocks, 128, split_pair_smem(WAVE, d.Ls, buffers), s>>>(d, p, buffers);
-#else
-    split_eval32<WAVE><<<sms * 16, 128, 0, s>>>(d, p);
-#endif
     if (!e->capturing && cudaEventRecord(e->sp_ev[2 * r + 1], s) != cudaSuccess) return -1;
     split_redo<WAVE><<<redo_blocks, 128, 0, s>>>(d, p);
     split_book<WAVE><<<book_blocks, 128, 0, s>>>(d, p);

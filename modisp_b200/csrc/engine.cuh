@@ -53,7 +53,7 @@ enum Counter {
 };
 
 struct ScanState;
-struct SplitSample;
+struct SplitRound;
 struct SplitTrace;
 
 struct Dev {
@@ -121,7 +121,7 @@ struct Dev {
   int sp_cap;           // active-set capacity (traces)
   int *sp_act[2];       // active trace lists by round parity
   ScanState *sp_state;  // [n_traces] scan state between rounds
-  struct SplitSample *sp_s;  // [sp_cap][SPLIT_SAMPLES] samples of the round
+  struct SplitRound *sp_s;  // [sp_cap] samples of the round
   struct SplitTrace *sp_tr;  // [sp_cap] the active traces' evaluation constants
   int *sp_kf;           // [n_traces] knot interval of the trace's next grid point (a lower bound)
   int *sp_redo;         // samples to evaluate in FP64

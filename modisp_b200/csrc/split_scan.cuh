@@ -10,12 +10,10 @@
 //   split_positions        one warp per trace: the next SPLIT_STEPS steps'
 //                          positions, merged exactly as the fused scan merges
 //                          them (scan_positions, scan_position32)
-//   split_eval32           one thread per sample: the FP32 secular value; the
-//                          near-cutoff band takes the trace's FP64 tail values;
-//                          sign-uncertain samples are listed for FP64
-//   split_eval32_pair      Rayleigh: the same with one thread per two samples of
-//                          a trace, evaluated together in paired FP32
-//                          instructions (sm_100 .f32x2)
+//   split_eval32_pair      one thread per two samples of a trace, evaluated
+//                          together in paired FP32 instructions (sm_100 .f32x2);
+//                          the near-cutoff band takes the trace's FP64 tail
+//                          values; sign-uncertain samples are listed for FP64
 //   split_redo             one thread per listed sample: its FP64 value
 //   split_book             one thread per trace: the samples in order through
 //                          the fused scan's bookkeeping (sign changes, regular
@@ -38,23 +36,11 @@
 namespace md200 {
 
 // Compile-time tuning: 32-sample steps per trace per round (two measured best:
-// fewer samples evaluated past a trace's last bracket than four, half the
-// rounds of one); the evaluation kernel's minimum resident CTAs per SM (1: no
-// register cap; capping it measured no faster); Rayleigh values two samples
-// per thread in paired FP32 instructions (split_eval32_pair, on with two steps
-// per round), that kernel's minimum resident CTAs per SM (4: 122 registers,
-// no spills; uncapped, 138 registers and 3 CTAs ran 13 % slower, 5 CTAs spill)
-// and its grid in CTAs per SM (64: 2.4 % faster than 16, 128 no faster; the
-// grid-stride loop then takes a few pairs per thread).
-#ifndef MD200_SPLIT_STEPS
-#define MD200_SPLIT_STEPS 2
-#endif
-#ifndef MD200_SPLIT_EVAL_BLOCKS
-#define MD200_SPLIT_EVAL_BLOCKS 1
-#endif
-#ifndef MD200_SPLIT_PAIR
-#define MD200_SPLIT_PAIR (MD200_SPLIT_STEPS == 2)
-#endif
+// fewer samples evaluated past a trace's last bracket than four, half the rounds of
+// one; the paired evaluation takes one sample of each); the evaluation kernel's
+// minimum resident CTAs per SM (Rayleigh 4: 128 registers; 3 CTAs ran 10 % slower,
+// 5 CTAs 2 %.  Love 6: 8 ran 3 % slower, 5 the same) and its grid in CTAs per SM
+// (64: 2.4 % faster than 16, 128 no faster; a warp then takes a few traces).
 #ifndef MD200_SPLIT_PAIR_BLOCKS
 #define MD200_SPLIT_PAIR_BLOCKS 4
 #endif
@@ -64,7 +50,7 @@ namespace md200 {
 #ifndef MD200_SPLIT_PAIR_GRID
 #define MD200_SPLIT_PAIR_GRID 64
 #endif
-constexpr int SPLIT_STEPS = MD200_SPLIT_STEPS;    // 32-sample steps per trace per round
+constexpr int SPLIT_STEPS = 2;                    // 32-sample steps per trace per round
 constexpr int SPLIT_SAMPLES = 32 * SPLIT_STEPS;  // sample slots per active trace
 constexpr int SPLIT_ACTIVE_MAX = 1 << 20;         // active-set capacity (traces)
 // Runs with fewer traces use the fused kernel.  Scan stage, fused against split:
@@ -77,15 +63,20 @@ constexpr int ZOOM_TROUGH = 0, ZOOM_LAST = 1;
 
 }  // namespace md200
 
-// One sample of a round: position, secular value, shape feature and
-// log-magnitude, bits (seed, near cutoff, FP64 value).  32 bytes, one memory
-// sector: the bookkeeping thread of a trace reads its samples one sector each.
-// The trough tests and windows take the shape feature and log-magnitude in
-// single precision only, so float keeps every decision of the fused scan.
-struct md200::SplitSample {
-  double c, F;
-  float g, M;
-  unsigned k, pad;
+// One trace's samples of a round: positions, FP32 secular values, shape features
+// and log-magnitudes, bits (seed, near cutoff, FP64 value), and the FP64 values of
+// the samples that have one.  By field, so that a warp's stores and loads of 32
+// slots are whole sectors and the bookkeeping thread fetches four samples' fields
+// 16 bytes at a time.  (As 32-byte records every field of every slot was a sector
+// of its own: scan stage of 20,000 models, Love 17.2 -> 16.8 ms, Rayleigh 36.9 ->
+// 36.4.)  The trough tests and windows take the shape feature and
+// log-magnitude in single precision only, and of an FP32 value the bookkeeping
+// takes the sign, so float keeps every decision of the fused scan.
+struct md200::SplitRound {
+  double c[md200::SPLIT_SAMPLES];
+  float F[md200::SPLIT_SAMPLES], g[md200::SPLIT_SAMPLES], M[md200::SPLIT_SAMPLES];
+  unsigned k[md200::SPLIT_SAMPLES];
+  double F64[md200::SPLIT_SAMPLES];
 };
 
 // An active trace's constants for the evaluation threads, written by its
@@ -96,7 +87,7 @@ struct md200::SplitTrace {
 };
 
 namespace md200 {
-static_assert(sizeof(SplitSample) == 32, "one sector per sample");
+static_assert(sizeof(SplitRound) % 16 == 0 && SPLIT_SAMPLES % 4 == 0, "16-byte copies of four samples");
 
 // Warp-aggregated append: every lane of the warp calls it (n = 0 where there is
 // nothing to add); returns this lane's base index in the list behind `counter`.
@@ -187,7 +178,7 @@ __global__ void __launch_bounds__(128) split_positions(Dev d, int p) {
       tr.pad0 = tr.pad1 = 0;
       d.sp_tr[i] = tr;
     }
-    SplitSample *ss = d.sp_s + static_cast<size_t>(i) * SPLIT_SAMPLES;
+    SplitRound &ss = d.sp_s[i];
     bool done = false;
     for (int s = 0; s < SPLIT_STEPS; ++s) {
       double c = INFINITY;
@@ -204,73 +195,28 @@ __global__ void __launch_bounds__(128) split_positions(Dev d, int p) {
         scan_position32(c, x.hi, near_cut);
         k = ((seeds >> lane) & 1u ? SK_SEED : 0u) | (near_cut ? SK_NEAR : 0u);
       }
-      ss[s * 32 + lane].c = c;
-      ss[s * 32 + lane].k = k;
+      ss.c[s * 32 + lane] = c;
+      ss.k[s * 32 + lane] = k;
     }
   }
 }
 
 // A near-cutoff sample: the trace's FP64 tail value when it is at this position
 // (returns false), else true (the sample goes to the FP64 list).
-__device__ __forceinline__ bool split_near(const Dev &d, int t, SplitSample &smp, double c, unsigned &k) {
+__device__ __forceinline__ bool split_near(const Dev &d, int t, SplitRound &smp, int j, double c, unsigned &k) {
   const double4 *tail = d.tail + 2 * static_cast<size_t>(t);
   const double4 t0 = tail[0], t1 = tail[1];
   const double4 tv = c == t0.x ? t0 : t1;
   if (c == tv.x && isfinite(tv.y)) {
-    smp.F = tv.y;
-    smp.g = static_cast<float>(tv.z);
-    smp.M = static_cast<float>(tv.w);
+    smp.F64[j] = tv.y;
+    smp.g[j] = static_cast<float>(tv.z);
+    smp.M[j] = static_cast<float>(tv.w);
     k |= SK_EXACT;
     return false;
   }
   return true;
 }
 
-// One thread per sample slot: the FP32 value (the fused scan's scan_eval call on
-// the same single-precision position), or the trace's FP64 tail value in the
-// near-cutoff band; samples the FP32 value leaves sign-uncertain, and near-cutoff
-// samples without a tail value, are listed for FP64 (scan_complete32's rule).
-template <int WAVE>
-__global__ void __launch_bounds__(128, MD200_SPLIT_EVAL_BLOCKS) split_eval32(Dev d, int p) {
-  const int lane = threadIdx.x & 31;
-  const long long n = static_cast<long long>(d.ctr[C_SP_ACT0 + p]) * SPLIT_SAMPLES;
-  const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
-  unsigned long long steps = 0;  // FP32 layer steps evaluated here (MD200_STAT_SPLIT_EVAL_STEPS)
-  // the loop runs whole warps (n is a multiple of 32), so appends are warp-wide
-  for (long long q = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; q < n; q += stride) {
-    const int i = static_cast<int>(q / SPLIT_SAMPLES);
-    SplitSample &smp = d.sp_s[q];
-    const double c = smp.c;
-    unsigned k = smp.k;
-    bool redo = false;
-    if (c < INFINITY) {
-      const SplitTrace tr = d.sp_tr[i];
-      if (k & SK_NEAR) {
-        redo = split_near(d, tr.t, smp, c, k);
-      } else {
-        const LayerView<float> view = make_view<float>(layer_table<float>(d, tr.b), d.Ls, tr.L, tr.water);
-        const float c32 = static_cast<float>(c);
-        float F32, g32, M32;
-        scan_eval<float, WAVE, 1>(view, static_cast<float>(tr.w), &c32, &F32, &g32, &M32);
-        steps += layer_steps(tr.L, tr.water);
-        const double g = g32;
-        smp.F = F32;
-        smp.g = g32;
-        smp.M = M32;
-        redo = !(fabs(g) > MD200_REDO_G);
-      }
-      if (!redo) smp.k = k;
-    }
-    const int at = warp_append(&d.ctr[C_SP_REDO], redo ? 1 : 0, lane);
-    if (redo) d.sp_redo[at] = static_cast<int>(q);
-  }
-  if (d.stats) {
-    for (int o = 16; o; o >>= 1) steps += __shfl_xor_sync(FULL, steps, o);
-    if (lane == 0 && steps) atomicAdd(&d.stats[19], steps);
-  }
-}
-
-#if MD200_SPLIT_PAIR
 // One thread per pair of sample slots of an active trace -- slot j of its first
 // 32-sample step and slot j of its second -- whose FP32 values come from one paired
 // evaluation (rayleigh_eval32<R2>, love_eval32<R2>: each half bit for bit the
@@ -324,16 +270,16 @@ __global__ void __launch_bounds__(128, WAVE ? MD200_SPLIT_PAIR_BLOCKS_LOVE : MD2
     }
     __syncwarp();
     const int i = static_cast<int>(q >> 5);
-    const long long q0 = static_cast<long long>(i) * SPLIT_SAMPLES + (q & 31), q1 = q0 + 32;
-    SplitSample &s0 = d.sp_s[q0], &s1 = d.sp_s[q1];
-    const double c0 = s0.c, c1 = s1.c;
-    unsigned k0 = s0.k, k1 = s1.k;
+    const int j0 = static_cast<int>(q & 31), j1 = j0 + 32;
+    SplitRound &smp = d.sp_s[i];
+    const double c0 = smp.c[j0], c1 = smp.c[j1];
+    unsigned k0 = smp.k[j0], k1 = smp.k[j1];
     bool redo0 = false, redo1 = false;
     if (c0 < INFINITY || c1 < INFINITY) {
       const SplitTrace tr = d.sp_tr[i];
       const bool e0 = c0 < INFINITY && !(k0 & SK_NEAR), e1 = c1 < INFINITY && !(k1 & SK_NEAR);
-      if (c0 < INFINITY && !e0) redo0 = split_near(d, tr.t, s0, c0, k0);
-      if (c1 < INFINITY && !e1) redo1 = split_near(d, tr.t, s1, c1, k1);
+      if (c0 < INFINITY && !e0) redo0 = split_near(d, tr.t, smp, j0, c0, k0);
+      if (c1 < INFINITY && !e1) redo1 = split_near(d, tr.t, smp, j1, c1, k1);
       if (e0 || e1) {
         const LayerView<float> view = make_view<float>(layer_table<float>(d, tr.b), d.Ls, tr.L, tr.water);
         const float w = static_cast<float>(tr.w);
@@ -344,34 +290,33 @@ __global__ void __launch_bounds__(128, WAVE ? MD200_SPLIT_PAIR_BLOCKS_LOVE : MD2
         else rayleigh_eval32<R2>(Layers2{view, mine + buf * n16}, kk, make_float2(w / kk.x, w / kk.y), w, &F, &g, &M);
         const unsigned long long ls = layer_steps(tr.L, tr.water);
         if (e0) {
-          s0.F = F.x;
-          s0.g = g.x;
-          s0.M = M.x;
+          smp.F[j0] = F.x;
+          smp.g[j0] = g.x;
+          smp.M[j0] = M.x;
           redo0 = !(fabs(static_cast<double>(g.x)) > MD200_REDO_G);
           steps += ls;
         }
         if (e1) {
-          s1.F = F.y;
-          s1.g = g.y;
-          s1.M = M.y;
+          smp.F[j1] = F.y;
+          smp.g[j1] = g.y;
+          smp.M[j1] = M.y;
           redo1 = !(fabs(static_cast<double>(g.y)) > MD200_REDO_G);
           steps += ls;
         }
       }
-      if (c0 < INFINITY && !redo0) s0.k = k0;
-      if (c1 < INFINITY && !redo1) s1.k = k1;
+      if (c0 < INFINITY && !redo0) smp.k[j0] = k0;
+      if (c1 < INFINITY && !redo1) smp.k[j1] = k1;
     }
     __syncwarp();  // the records are read: their buffer may be filled again
     int at = warp_append(&d.ctr[C_SP_REDO], (redo0 ? 1 : 0) + (redo1 ? 1 : 0), lane);
-    if (redo0) d.sp_redo[at++] = static_cast<int>(q0);
-    if (redo1) d.sp_redo[at] = static_cast<int>(q1);
+    if (redo0) d.sp_redo[at++] = i * SPLIT_SAMPLES + j0;
+    if (redo1) d.sp_redo[at] = i * SPLIT_SAMPLES + j1;
   }
   if (d.stats) {
     for (int o = 16; o; o >>= 1) steps += __shfl_xor_sync(FULL, steps, o);
     if (lane == 0 && steps) atomicAdd(&d.stats[19], steps);
   }
 }
-#endif  // MD200_SPLIT_PAIR
 
 // One thread per listed sample: its FP64 value (eval64_outline, as in the fused
 // scan).
@@ -381,14 +326,14 @@ __global__ void __launch_bounds__(128) split_redo(Dev d, int p) {
   for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
     const int q = d.sp_redo[r];
     const SplitTrace tr = d.sp_tr[q / SPLIT_SAMPLES];
-    SplitSample &smp = d.sp_s[q];
+    SplitRound &smp = d.sp_s[q / SPLIT_SAMPLES];
+    const int j = q % SPLIT_SAMPLES;
     double g, M;
-    const double F = eval64_outline(make_view<double>(layer_table<double>(d, tr.b), d.Ls, tr.L, tr.water), WAVE,
-                                    tr.w, smp.c, &g, &M);
-    smp.F = F;
-    smp.g = static_cast<float>(g);
-    smp.M = static_cast<float>(M);
-    smp.k |= SK_EXACT | SK_REDO;
+    smp.F64[j] = eval64_outline(make_view<double>(layer_table<double>(d, tr.b), d.Ls, tr.L, tr.water), WAVE, tr.w,
+                                smp.c[j], &g, &M);
+    smp.g[j] = static_cast<float>(g);
+    smp.M[j] = static_cast<float>(M);
+    smp.k[j] |= SK_EXACT | SK_REDO;
   }
 }
 
@@ -421,10 +366,11 @@ __device__ __forceinline__ bool needs_last_cell(const ScanState &st, int K) {
   return u > v + noise && v / ((u - v) / h0) < 1.25f * h0;
 }
 
-// Records a bookkeeping thread has on their way to shared memory: the loop is a
-// chain of dependent decisions, its loads need not be.  (One ahead, in registers,
-// it waited 8 warps an issue for memory.)
-constexpr int BOOK_AHEAD = 4;
+// The bookkeeping loop is a chain of dependent decisions, its loads need not be: each
+// thread has the next four samples' fields on their way to shared memory while it
+// works on four (one sample ahead, in registers, it waited 8 warps an issue for
+// memory).
+constexpr int BOOK_FIELDS = 6;  // 16-byte pieces of four samples: c (2), F, g, M, k
 
 // One thread per active trace: its samples of this round in order, through the
 // bookkeeping of scan_bookkeep (one lane's share of it, carried sample by
@@ -434,17 +380,21 @@ constexpr int BOOK_AHEAD = 4;
 template <int WAVE>
 __global__ void __launch_bounds__(128) split_book(Dev d, int p) {
   constexpr bool single = true;
-  __shared__ float4 ring[2][BOOK_AHEAD][128];
+  __shared__ float4 ring[2][BOOK_FIELDS][128];
   const int lane = threadIdx.x & 31;
   const int n = d.ctr[C_SP_ACT0 + p];
   const int stride = gridDim.x * blockDim.x;
   const int n_pad = (n + 31) & ~31;
-  // record j of a trace's samples into this thread's ring
-  auto fetch = [&](const SplitSample *rec, int j) {
-    if (j < SPLIT_SAMPLES) {
-      const float4 *src = reinterpret_cast<const float4 *>(rec + j);
-      cp_async16(&ring[0][j % BOOK_AHEAD][threadIdx.x], src);
-      cp_async16(&ring[1][j % BOOK_AHEAD][threadIdx.x], src + 1);
+  // samples 4 grp .. 4 grp + 3 of a trace into this thread's places
+  auto fetch = [&](const SplitRound &r, int grp) {
+    if (grp < SPLIT_SAMPLES / 4) {
+      float4(&to)[BOOK_FIELDS][128] = ring[grp & 1];
+      cp_async16(&to[0][threadIdx.x], &r.c[4 * grp]);
+      cp_async16(&to[1][threadIdx.x], &r.c[4 * grp + 2]);
+      cp_async16(&to[2][threadIdx.x], &r.F[4 * grp]);
+      cp_async16(&to[3][threadIdx.x], &r.g[4 * grp]);
+      cp_async16(&to[4][threadIdx.x], &r.M[4 * grp]);
+      cp_async16(&to[5][threadIdx.x], &r.k[4 * grp]);
     }
     asm volatile("cp.async.commit_group;\n" ::);
   };
@@ -463,34 +413,29 @@ __global__ void __launch_bounds__(128) split_book(Dev d, int p) {
       st = d.sp_state[t];
       K = d.tr_modes[t] + 2;
       double *slot = d.slot + static_cast<size_t>(t) * d.KB * SLOT;
-      const size_t base = static_cast<size_t>(i) * SPLIT_SAMPLES;
+      const SplitRound &round = d.sp_s[i];
       const SplitTrace tr = d.sp_tr[i];
       const unsigned long long nsteps = layer_steps(tr.L, tr.water);
       bool stop = false;  // the K-th bracket, the window end or a non-finite value
-      for (int j = 0; j < BOOK_AHEAD; ++j) fetch(d.sp_s + base, j);
+      fetch(round, 0);
       for (int j = 0; j < SPLIT_SAMPLES; ++j) {
-        asm volatile("cp.async.wait_group %0;\n" ::"n"(BOOK_AHEAD - 1) : "memory");
-        SplitSample smp;
-        {
-          const float4 a = ring[0][j % BOOK_AHEAD][threadIdx.x], b = ring[1][j % BOOK_AHEAD][threadIdx.x];
-          smp.c = __hiloint2double(__float_as_int(a.y), __float_as_int(a.x));
-          smp.F = __hiloint2double(__float_as_int(a.w), __float_as_int(a.z));
-          smp.g = b.x;
-          smp.M = b.y;
-          smp.k = __float_as_uint(b.z);
+        if ((j & 3) == 0) {
+          fetch(round, j / 4 + 1);
+          asm volatile("cp.async.wait_group 1;\n" ::: "memory");
         }
-        fetch(d.sp_s + base, j + BOOK_AHEAD);
-        const double c = smp.c;
+        const float4(&at)[BOOK_FIELDS][128] = ring[(j >> 2) & 1];
+        auto field = [&](int q) { return reinterpret_cast<const float *>(&at[q][threadIdx.x])[j & 3]; };
+        const double c = reinterpret_cast<const double *>(&at[(j & 3) >> 1][threadIdx.x])[j & 1];
         if (!(c < INFINITY)) {  // the window is exhausted
           st.bits |= SS_FINISHED;
           stop = true;
           break;
         }
-        const double F = smp.F;
-        const float gf = smp.g, Mf = smp.M;
-        const double g = gf;
-        const unsigned k = smp.k;
+        const unsigned k = __float_as_uint(field(5));
         const bool exact = (k & SK_EXACT) != 0;
+        const double F = exact ? round.F64[j] : static_cast<double>(field(2));
+        const float gf = field(3), Mf = field(4);
+        const double g = gf;
         ++ev32;
         sts32 += nsteps;
         ev += (k & SK_REDO) ? 2 : 1;
