@@ -85,12 +85,6 @@ __device__ __noinline__ void scan_eval(const LayerView<T> view, T w, const T *c,
 // Layer recurrence steps of one evaluation.
 __device__ __forceinline__ int layer_steps(int L, int water) { return L - 1 - water; }
 
-// FP64 secular value (and shape feature) from a global-memory table.
-__device__ __forceinline__ double eval64(const LayerView<double> &m, int wave, double w, double c,
-                                         double *g) {
-  return secular<double, double>(m, wave, w / c, w, g);
-}
-
 // Out-of-line FP64 evaluation for the rare FP64 re-evaluations inside the FP32
 // scan, so their registers do not weigh on the single-precision loop.
 __device__ __noinline__ double eval64_outline(const LayerView<double> &m, int wave, double w, double c,
@@ -559,12 +553,15 @@ __global__ void init_traces(Dev d) {
 // FP64 values at the two near-cutoff positions of every trace, for the FP32
 // scan (one thread per trace, all lanes busy): near the half-space cutoff the
 // start vector depends on the small radical sqrt(k^2 - kb^2) directly, which
-// single precision resolves poorly.
+// single precision resolves poorly.  Traces in model order: a warp's periods share
+// one model, its layer count and every branch (in the order of the trace list, a
+// model each, 20,000 models x 60 periods took 0.95 ms against 0.70, Love 0.55 against
+// 0.30).
 __global__ void tail_values(Dev d) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= *(volatile int *)&d.ctr[C_NTRACE]) return;
-  const int t = d.trace_list[q];
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= d.n_traces) return;
   const int b = d.tr_model[t];
+  if (d.mstate[b] != 0 || (d.crole && d.crole[t] == 2)) return;  // not scanned
   const double w = TWO_PI / d.tr_period[t];
   const LayerView<double> m = make_view<double>(d.layer64 + static_cast<size_t>(b) * ROWS * d.Ls, d.Ls,
                                                 d.mL[b], d.mwater[b]);
@@ -1845,7 +1842,8 @@ __global__ void assemble(Dev d, const int *list = nullptr, int count_id = 0) {
     double root = mo < n ? r(mo) : NAN;
     if (isfinite(root) && root >= .99 * vs_hs) fl |= TRACE_NEAR_CUTOFF;
     if (isfinite(root) && d.accept < 1.) {
-      const double v = eval64(m, d.wave, w, root, nullptr);
+      double g, lm;
+      const double v = eval64_outline(m, d.wave, w, root, &g, &lm);
       if (!isfinite(v) || fabs(v) > d.accept) {
         root = NAN;
         fl |= TRACE_F_REJECTED;
@@ -1879,11 +1877,17 @@ __global__ void assemble(Dev d, const int *list = nullptr, int count_id = 0) {
   d.olevels[t] = level;
   d.ocounts[t] = count;
   if (d.stats) {
-    if (!list) atomicAdd(&d.stats[11], 1ULL);
-    if (failed) atomicAdd(&d.stats[8], 1ULL);
     int finite = 0;
     for (int mo = 0; mo < nm && mo < n; ++mo) finite += isfinite(d.vel[out0 + static_cast<size_t>(mo) * T]);
-    if (finite) atomicAdd(&d.stats[10], static_cast<unsigned long long>(finite));
+    // one addition a warp: every trace adding for itself made two thirds of the kernel
+    const unsigned here = __activemask();
+    const unsigned roots = __reduce_add_sync(here, static_cast<unsigned>(finite));
+    const unsigned lost = __popc(__ballot_sync(here, failed));
+    if ((threadIdx.x & 31) == __ffs(here) - 1) {
+      if (!list) atomicAdd(&d.stats[11], static_cast<unsigned long long>(__popc(here)));
+      if (lost) atomicAdd(&d.stats[8], static_cast<unsigned long long>(lost));
+      if (roots) atomicAdd(&d.stats[10], static_cast<unsigned long long>(roots));
+    }
   }
 }
 
