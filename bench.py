@@ -63,17 +63,17 @@ WORKLOAD = ("mixed-precision batch: 100000 models x 8-20 layers, 30 % with one l
 FLOPS_PER_STEP = {0: 170, 1: 24}
 # DRAM traffic of the split scan's Rayleigh evaluation kernel (split_eval32_pair) per
 # FP32 layer step it evaluates: dram__bytes_read.sum + dram__bytes_write.sum over
-# the 9 launches of one run (1,090.4 MB + 715.8 MB), from an ncu capture of 2,000
+# the 4 launches of one run (358.7 MB + 215.1 MB), from an ncu capture of 2,000
 # mixed-precision models, divided by that run's evaluated layer steps
-# (MD200_STAT_SPLIT_EVAL_STEPS, 437,558,855).
-EVAL_DRAM_BYTES_PER_STEP = (1090352896 + 715775488) / 437558855
+# (MD200_STAT_SPLIT_EVAL_STEPS, 343,048,695).
+EVAL_DRAM_BYTES_PER_STEP = (358701312 + 215132672) / 343048695
 
 
 def split_rounds(n_traces):
     """Launches of the split scan's evaluation kernel in one run (the engine's
-    split_rounds: an active set of up to 2^20 traces, 3 rounds per set + 6)."""
+    split_rounds for Rayleigh: an active set of up to 2^20 traces, 3 rounds per set + 1)."""
     cap = min(n_traces, 1 << 20)
-    return min(64, 3 * (-(-n_traces // cap)) + 6)
+    return min(64, 3 * (-(-n_traces // cap)) + 1)
 
 
 def parse():
@@ -861,8 +861,8 @@ def main():
                                              "chosen_by": ("engine defaults (--no-autotune)" if args.no_autotune else
                                                            "autotuner on 1,000 of the models, both waves") +
                                                           ": fused-scan warps per CTA, CTAs per SM, FP32 scan form "
-                                                          "(0 automatic: split rounds for Rayleigh, fused for Love; "
-                                                          "1 fused; 2 split)"}},
+                                                          "(0 automatic, by the run's traces; 1 fused; "
+                                                          "2 split rounds)"}},
             "fp64": {"value": value64, "unit": "roots/s", "ms_per_step": ms64 / args.steps,
                      "fp32_scan_speedup": value / value64,
                      "stage_ms": {("rayleigh" if w == 0 else "love"): stage64[w] for w in (0, 1)}},
@@ -882,15 +882,14 @@ def main():
                                               "functions not counted",
                          "traffic_note": "DRAM bytes per evaluated layer step from an ncu capture of every "
                                          "evaluation launch of a 2,000-model run, times this launch's steps; the "
-                                         "kernel reads 32-byte sample records and the model tables and is "
-                                         "compute-bound",
+                                         "kernel reads and writes the samples' fields and the models' layer "
+                                         "records and is compute-bound",
                          "peak_kind": "measured FMA throughput (md200_measure_peak), not MEASURED_PEAKS.json",
                          "fp64_peak": peak64 / 1e12,
                          "scan_stage": {"achieved": scan_achieved / 1e12, "frac": scan_achieved / peak32,
                                         "ms_per_step": scan_ms,
-                                        "note": "the whole FP32 scan stage of both waves (split rounds for "
-                                                "Rayleigh, fused kernel for Love), algorithmic flops of the "
-                                                "samples the scans consumed"},
+                                        "note": "the whole FP32 scan stage of both waves, algorithmic flops of "
+                                                "the samples the scans consumed"},
                          "stage_ms": {("rayleigh" if w == 0 else "love"): stage[w] for w in (0, 1)}},
             "cpu_baseline": cpu,
             "cpu_baseline_auto": cpu_auto,

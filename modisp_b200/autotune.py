@@ -5,10 +5,10 @@ depth, the period range and the wave: warps per CTA (1, 2 or 4 traces in flight
 per CTA) and the number of resident CTAs per SM trade latency hiding against
 instruction-cache and register pressure.  The FP32-scan engine also has two
 forms of its scan, which put a different number of threads on a trace: the fused
-kernel (one warp per trace) and the split rounds (one thread per sample for the
-values, one thread per trace for the bookkeeping, one warp per trace for the
-positions); the candidates cover both, and the automatic choice (split for
-Rayleigh, fused for Love).  ``autotune`` times each candidate on a sample of the
+kernel (one warp per trace) and the split rounds (one thread per two samples for
+the values, one thread per trace for the bookkeeping, one warp per trace for the
+positions); the candidates cover both, and the automatic choice (split from 16,384
+Rayleigh or 131,072 Love traces on).  ``autotune`` times each candidate on a sample of the
 caller's workload (device time of full runs, best of ``repeats``; both waves
 when ``wave`` is None), checks that every candidate returns bit-identical
 results (neither the launch shape nor the scan form may change a root), and
@@ -33,7 +33,7 @@ from . import _native
 # (warps per CTA, CTAs per SM; 0 = as many as registers allow) of the fused scan
 SHAPES = ((4, 0), (4, 3), (4, 2), (2, 0), (2, 4), (1, 0))
 # scan forms of the FP32-scan engine (md200_options.scan_mode): 0 automatic
-# (split rounds for Rayleigh, fused kernel for Love), 1 fused, 2 split
+# (by wave and number of traces), 1 fused, 2 split
 FP32_MODES = (0, 1, 2)
 
 
