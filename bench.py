@@ -71,7 +71,7 @@ EVAL_DRAM_BYTES_PER_STEP = (358701312 + 215132672) / 343048695
 
 def split_rounds(n_traces):
     """Launches of the split scan's evaluation kernel in one run (the engine's
-    split_rounds for Rayleigh: an active set of up to 2^20 traces, 3 rounds per set + 1)."""
+    split_rounds for Rayleigh and 5 modes: an active set of up to 2^20 traces, 3 rounds per set + 1)."""
     cap = min(n_traces, 1 << 20)
     return min(64, 3 * (-(-n_traces // cap)) + 1)
 

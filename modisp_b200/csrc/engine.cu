@@ -383,10 +383,13 @@ constexpr int MODEL_LIST_MIN_TRACES = 4096;
 // unfinished after them are handed to the fused kernel.  A round of nothing costs
 // 35-40 us of launches, a handed-over trace a warp's scan of its rest.  Measured best
 // at 3, 120 and 1,200 thousand traces: 3 (Love) and 4 rounds (Rayleigh) per
-// active set; with nine, 120,000 Rayleigh traces took 4.41 ms against 4.16.
-int split_rounds(int nt, int cap, int wave) {
+// active set; with nine, 120,000 Rayleigh traces took 4.41 ms against 4.16.  More
+// modes take a Rayleigh trace more rounds, and what the rounds leave costs the fused
+// kernel more: one round for every four brackets past seven (180,000 traces of ten
+// modes: 4 rounds 8.05 ms, 5 7.51, 9 7.6; 40,000 of a hundred modes: 4 14.6, 27 13.2).
+int split_rounds(int nt, int cap, int wave, int K) {
   const int waves = (nt + cap - 1) / cap;
-  return std::min(md200_engine::MAX_SPLIT_ROUNDS, 3 * waves + (wave == 0 ? 1 : 0));
+  return std::min(md200_engine::MAX_SPLIT_ROUNDS, 3 * waves + (wave == 0 ? 1 + std::max(0, K - 7) / 4 : 0));
 }
 
 // The split FP32 scan's launches (split_scan.cuh): `rounds` rounds, then the
@@ -515,7 +518,7 @@ int enqueue(md200_engine *e, const double *h, const double *vp, const double *vs
   const bool split = d.fp32 && (e->o.scan_mode == 2 ||
                                 (e->o.scan_mode == 0 && nt >= SPLIT_MIN_TRACES[wave]));
   if (split) {
-    const int rounds = split_rounds(nt, d.sp_cap, wave);
+    const int rounds = split_rounds(nt, d.sp_cap, wave, d.K);
     const int launched = wave == 0 ? split_scan<0>(e, dm, rounds, s) : split_scan<1>(e, dm, rounds, s);
     if (launched < 0) return fail("modisp_b200 CUDA: event record failed in the split scan");
     nl += launched;

@@ -480,7 +480,10 @@ __global__ void prep_models(Dev d, int sortcap, int bodycap, int tables) {
   //    window's lower end.  Below every body velocity N(c) = 0, so grid point j
   //    is the log point lo (hi/lo)^(j/nlog).
   const double cl = fmin(fmax(lowest_root(t64, Ls, L, wave, top, lane), lo), hi);
-  const int j0 = max(1, static_cast<int>(floor(log(cl / lo) * nlog / lspan)) - SCAN_START_MARGIN);
+  //    (A window so narrow that log points could coincide keeps its first.)
+  const int j0 = lspan > 1e-9
+                     ? max(1, static_cast<int>(floor(log(cl / lo) * nlog / lspan)) - SCAN_START_MARGIN)
+                     : 1;
   const double c0 = j0 > 1 ? lo * exp(lspan * j0 / nlog) : 0.;
   int ns = 0, s0 = 0;
   double *sd = d.seed + static_cast<size_t>(b) * d.nsmax;
