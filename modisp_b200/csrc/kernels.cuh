@@ -41,13 +41,22 @@ __device__ __forceinline__ unsigned lanemask_lt() {
   return m;
 }
 
-// 16-byte asynchronous global->shared copy (Ampere+ cp.async, bypassing L1).
+// 16-byte asynchronous global->shared copies (Ampere+ cp.async, bypassing L1), their
+// groups and the waits for them.  Each is a compiler barrier too: a plain load of
+// the bytes a copy replaces must stay above it, a load of what it brings below the
+// wait.
 __device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
   const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem));
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int LEFT>  // groups that may still be on their way
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;\n" ::"n"(LEFT) : "memory");
 }
 __device__ __forceinline__ void cp_async_wait_all() {
-  asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::);
+  cp_async_commit();
+  cp_async_wait<0>();
 }
 
 template <class T>

@@ -253,7 +253,7 @@ __global__ void __launch_bounds__(128, WAVE ? MD200_SPLIT_PAIR_BLOCKS_LOVE : MD2
       const float4 *src = reinterpret_cast<const float4 *>(d.pair32) + static_cast<size_t>(d.sp_tr[q >> 5].b) * n16;
       for (int j = lane; j < n16; j += 32) cp_async16(mine + buf * n16 + j, src + j);
     }
-    asm volatile("cp.async.commit_group;\n" ::);
+    cp_async_commit();
   };
   unsigned long long steps = 0;
   int buf = 0;
@@ -263,10 +263,10 @@ __global__ void __launch_bounds__(128, WAVE ? MD200_SPLIT_PAIR_BLOCKS_LOVE : MD2
   for (long long q = first; q < n; q += stride, buf ^= buffers - 1) {
     if (buffers == 2) {
       stage(q + stride, buf ^ 1);
-      asm volatile("cp.async.wait_group 1;\n" ::);
+      cp_async_wait<1>();
     } else {
       stage(q, 0);
-      asm volatile("cp.async.wait_group 0;\n" ::);
+      cp_async_wait<0>();
     }
     __syncwarp();
     const int i = static_cast<int>(q >> 5);
@@ -396,7 +396,7 @@ __global__ void __launch_bounds__(128) split_book(Dev d, int p) {
       cp_async16(&to[4][threadIdx.x], &r.M[4 * grp]);
       cp_async16(&to[5][threadIdx.x], &r.k[4 * grp]);
     }
-    asm volatile("cp.async.commit_group;\n" ::);
+    cp_async_commit();
   };
   // counters of the samples the bookkeeping consumes, as the fused scan counts
   // its steps' samples: each an FP32 evaluation, the re-evaluated ones also FP64
@@ -421,7 +421,7 @@ __global__ void __launch_bounds__(128) split_book(Dev d, int p) {
       for (int j = 0; j < SPLIT_SAMPLES; ++j) {
         if ((j & 3) == 0) {
           fetch(round, j / 4 + 1);
-          asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+          cp_async_wait<1>();
         }
         const float4(&at)[BOOK_FIELDS][128] = ring[(j >> 2) & 1];
         auto field = [&](int q) { return reinterpret_cast<const float *>(&at[q][threadIdx.x])[j & 3]; };
@@ -527,7 +527,7 @@ __global__ void __launch_bounds__(128) split_book(Dev d, int p) {
         go_on = true;  // the round's samples are used up: more next round
       }
       d.sp_state[t] = st;
-      asm volatile("cp.async.wait_all;\n" ::: "memory");  // (the next trace's records take the same places)
+      cp_async_wait<0>();  // (the next trace's records take the same places)
     }
     split_publish(d, t, st, publish, lane);
     const int za = warp_append(&d.ctr[C_SP_ZOOM], zoom ? 1 : 0, lane);
