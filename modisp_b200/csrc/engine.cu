@@ -11,6 +11,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <new>
 #include <string>
 #include <thread>
@@ -226,6 +227,21 @@ size_t scan_smem(int warps, int Ls, size_t elem) {
   return static_cast<size_t>(warps) * (tab + 32 * sizeof(double));
 }
 
+// Room for `bytes` of dynamic shared memory in launches of `kernel` on the current
+// device.  The limit belongs to the kernel and holds for every engine of the
+// process, and a launch above it fails: it is raised, never lowered, or an engine
+// would lose its launches to the next one with smaller blocks.
+template <class... Args>
+int allow_shared(void (*kernel)(Args...), size_t bytes) {
+  static std::mutex lock;
+  const std::lock_guard<std::mutex> hold(lock);
+  cudaFuncAttributes now{};
+  MD200_CK(cudaFuncGetAttributes(&now, kernel));
+  if (bytes > static_cast<size_t>(now.maxDynamicSharedSizeBytes))
+    MD200_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)));
+  return 0;
+}
+
 int setup(md200_engine *e, bool staging) {
   MD200_CK(cudaSetDevice(e->device));
   MD200_CK(cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking));
@@ -310,16 +326,11 @@ int setup(md200_engine *e, bool staging) {
   e->scan_warps = e->o.warps_per_block > 0 ? std::min(4, e->o.warps_per_block) : 4;
   e->scan_smem64 = scan_smem(e->scan_warps, d.Ls, sizeof(double));
   e->scan_smem32 = scan_smem(e->scan_warps, d.Ls, sizeof(float));
-  for (auto fn : {scan<double, 0>, scan<double, 1>})
-    MD200_CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  static_cast<int>(std::max<size_t>(e->scan_smem64, 1024))));
-  for (auto fn : {scan<float, 0>, scan<float, 1>})
-    MD200_CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  static_cast<int>(std::max<size_t>(e->scan_smem32, 1024))));
-  MD200_CK(cudaFuncSetAttribute(split_eval32_pair<0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                static_cast<int>(split_pair_smem(0, d.Ls, split_pair_buffers(0, d.Ls)))));
-  MD200_CK(cudaFuncSetAttribute(split_eval32_pair<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                static_cast<int>(split_pair_smem(1, d.Ls, split_pair_buffers(1, d.Ls)))));
+  if (allow_shared(scan<double, 0>, e->scan_smem64) || allow_shared(scan<double, 1>, e->scan_smem64) ||
+      allow_shared(scan<float, 0>, e->scan_smem32) || allow_shared(scan<float, 1>, e->scan_smem32) ||
+      allow_shared(split_eval32_pair<0>, split_pair_smem(0, d.Ls, split_pair_buffers(0, d.Ls))) ||
+      allow_shared(split_eval32_pair<1>, split_pair_smem(1, d.Ls, split_pair_buffers(1, d.Ls))))
+    return 1;
   int occ64 = 0, occ32 = 0;
   MD200_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ64, scan<double, 0>, 32 * e->scan_warps,
                                                          e->scan_smem64));
@@ -346,9 +357,7 @@ int setup(md200_engine *e, bool staging) {
   for (auto &x : e->solved_ev) MD200_CK(cudaEventCreateWithFlags(&x, cudaEventDisableTiming));
   if (d.fp32)
     for (auto &x : e->sp_ev) MD200_CK(cudaEventCreate(&x));
-  MD200_CK(cudaFuncSetAttribute(prep_models, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                static_cast<int>(std::max<size_t>(e->prep_smem, 1024))));
-  return 0;
+  return allow_shared(prep_models, e->prep_smem);
 }
 
 // Lazily allocated engine-owned buffer.
