@@ -3,13 +3,14 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "brackets.cuh"
+
 namespace md200 {
 
 constexpr double TWO_PI = 6.283185307179586476925286766559;
 constexpr unsigned FULL = 0xffffffffu;
 constexpr int ROWS = 9;        // per-layer rows of the prepared table (7 used by the recurrence)
 constexpr int EVAL_ROWS = 7;   // rows staged into shared memory for the recurrence
-constexpr int SLOT = 5;        // doubles per bracket slot: lo, hi, flo, fhi, root
 constexpr long long JMAX = 1LL << 22;  // scan points per trace before the workspace flag (default)
 constexpr long long JMAX_FALLBACK = 1LL << 26;  // the fallback re-scan's limit
 

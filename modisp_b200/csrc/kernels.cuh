@@ -1603,21 +1603,13 @@ struct RefineLane {
   bool eval, exhausted, guard;
 };
 
-// Is bracket i of trace t a guard root (past the modes asked for) clear of every
-// other bracket by more than the close-root distance?  Its root is not reported:
-// it counts, keeps its rank, and decides whether a neighbour is close -- which its
-// bracket alone then settles, so it is confirmed but not refined.  Two of seven
-// brackets with five modes, a seventh (FP32 scan) to a quarter of refinement's
+// Is bracket i of trace t that of a guard root (past the modes asked for) which its
+// bracket alone settles (guard_is_clear)?  It is confirmed but not refined.  Two of
+// seven brackets with five modes, a seventh (FP32 scan) to a quarter of refinement's
 // evaluations.  (Anchor continuation reads guard roots.)
 __device__ __forceinline__ bool guard_settled(const Dev &d, int t, int i) {
   if (d.crole || i < d.tr_modes[t]) return false;
-  const double *sl = d.slot + static_cast<size_t>(t) * d.KB * SLOT;
-  const double lo = sl[static_cast<size_t>(i) * SLOT], hi = sl[static_cast<size_t>(i) * SLOT + 1];
-  for (int j = 0; j < d.nbr[t]; ++j) {
-    const double l = sl[static_cast<size_t>(j) * SLOT], h = sl[static_cast<size_t>(j) * SLOT + 1];
-    if (j < i ? !(lo - h > d.close_rtol * hi) : j > i && !(l - hi > d.close_rtol * h)) return false;
-  }
-  return true;
+  return guard_is_clear(d.slot + static_cast<size_t>(t) * d.KB * SLOT, d.nbr[t], i, d.close_rtol);
 }
 
 __device__ __forceinline__ void refine_step(Dev &d, RefineLane &L, double *x, unsigned long long &count) {
