@@ -32,4 +32,11 @@ MD200_BRACKET_FN bool guard_is_clear(const double *slots, int n, int i, double c
   return true;
 }
 
+// Do the FP64 values at a bracket's ends confirm it: finite, nonzero, of opposite
+// signs?  (Refinement fails a bracket with an infinite end, so its product of signs
+// must not settle one.)
+MD200_BRACKET_FN bool ends_confirm(double fa, double fb) {
+  return fa - fa == 0. && fb - fb == 0. && ((fa < 0. && fb > 0.) || (fa > 0. && fb < 0.));
+}
+
 }  // namespace md200

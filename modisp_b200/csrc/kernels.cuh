@@ -1614,7 +1614,7 @@ __device__ __forceinline__ bool guard_settled(const Dev &d, int t, int i) {
 
 __device__ __forceinline__ void refine_step(Dev &d, RefineLane &L, double *x, unsigned long long &count) {
   if (L.id < 0 || L.eval) return;
-  if (L.guard && !L.st.pending && L.st.sa.F * L.st.sb.F < 0.) {
+  if (L.guard && !L.st.pending && ends_confirm(L.st.sa.F, L.st.sb.F)) {
     L.sl[4] = .5 * (L.st.a + L.st.b);
     ++count;
     L.id = -1;

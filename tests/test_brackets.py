@@ -17,6 +17,7 @@ SOURCE = """
 extern "C" int clear_of(const double *slots, int n, int i, double rtol) {
   return md200::guard_is_clear(slots, n, i, rtol);
 }
+extern "C" int confirm(double fa, double fb) { return md200::ends_confirm(fa, fb); }
 """
 RTOL = .005
 
@@ -31,6 +32,7 @@ def rules(tmp_path_factory):
                     "-o", str(folder / "rules.so"), str(folder / "rules.cpp")], check=True)
     lib = ctypes.CDLL(str(folder / "rules.so"))
     lib.clear_of.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_double]
+    lib.confirm.argtypes = [ctypes.c_double, ctypes.c_double]
     return lib
 
 
@@ -107,3 +109,12 @@ def test_settled_guards_never_reach_a_reported_rank(rules):
 
         assert report(roots) == report(kept)
     assert settled > 500 and shared > 100
+
+
+@pytest.mark.parametrize("fa,fb,expected", [
+    (-1., 1., True), (1., -1e-300, True), (-1e-300, 1e-300, True), (-1e300, 1e300, True),
+    (1., 1., False), (-1., -1., False), (0., 1., False), (-1., 0., False), (-0., 1., False),
+    (-np.inf, 1., False), (1., -np.inf, False), (-np.inf, np.inf, False), (np.nan, 1., False), (-1., np.nan, False)])
+def test_ends_that_settle_a_guard(rules, fa, fb, expected):
+    """A guard is settled where refinement would end on a root: an infinite end fails there."""
+    assert bool(rules.confirm(fa, fb)) is expected
