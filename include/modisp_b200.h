@@ -99,6 +99,12 @@ md200_engine *md200_create(int device, int capacity, int layers, int periods, in
 md200_engine *md200_create_device(int device, int capacity, int layers, int periods, int nmodes,
                                   const md200_options *options);
 
+/* Device bytes such an engine reserves when it is made (the Jacobian and ragged runs
+ * of host arrays add buffers of their own on first use); -1 for an invalid geometry.
+ * Needs no device. */
+long long md200_workspace_bytes(int capacity, int layers, int periods, int nmodes,
+                                const md200_options *options);
+
 /* Replaces QeSolver.run(...) (cpp/cuda/qe.cu:1060-1119) with host arrays: copies
  * inputs to the device, solves, copies outputs back and synchronises.
  *   thickness, vp, vs, rho : [models, layers]

@@ -61,6 +61,7 @@ EXPORTS = {
     "md200_default_options": (None, [ctypes.POINTER(Options)]),
     "md200_create": (_P, [_I, _I, _I, _I, _I, ctypes.POINTER(Options)]),
     "md200_create_device": (_P, [_I, _I, _I, _I, _I, ctypes.POINTER(Options)]),
+    "md200_workspace_bytes": (ctypes.c_longlong, [_I, _I, _I, _I, ctypes.POINTER(Options)]),
     "md200_package": (_I, [_P, _I, _P, _P, _I, _I, _I, _D, _P, _P, _P, _P, _P, _P, _P, _P]),
     "md200_run": (_I, [_P, _P, _P, _P, _P, _I, _P, _P, _D, _D, _I, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _I]),
     "md200_run_device": (_I, [_P, _P, _P, _P, _P, _I, _P, _P, _D, _D, _I, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P,
@@ -412,6 +413,14 @@ def continuity_screen(periods, velocity, prediction=None, bilateral=True, device
     check(lib().md200_continuity_screen(int(device), ptr(p), T, ptr(v), B, K, ptr(pred), int(single),
                                         int(bool(bilateral)), ptr(flags), ctypes.byref(sus)))
     return flags, bool(sus.value)
+
+
+def workspace_bytes(capacity: int, layers: int, periods: int, nmodes: int, options: Options) -> int:
+    """Device bytes an engine of this geometry reserves (md200_workspace_bytes)."""
+    n = lib().md200_workspace_bytes(int(capacity), int(layers), int(periods), int(nmodes), ctypes.byref(options))
+    if n < 0:
+        raise RuntimeError(last_error())
+    return int(n)
 
 
 def package(velocity, flags, counts, close_rtol, group=None, group_flags=None):

@@ -207,15 +207,6 @@ def _models(thickness, vp, vs, rho):
     return arrays
 
 
-def _workspace_per_model(L, T, nmodes):
-    """Device bytes the engine reserves per model of capacity."""
-    K = nmodes + 2
-    KB = K + 16
-    per_trace = KB * 5 * 8 + 8 * 4 * 8 + KB * 4 + 8 * 4 + nmodes * (8 * 4 + 4 * 2 + 16) + 64
-    Ls = (L + 3) & ~3
-    return T * per_trace + 9 * Ls * 12 + (129 + 2 * L) * 32 + (6 * L + 32) * 8 + 96 + 4 * L * 8
-
-
 class Solver:
     """Reusable dispersion solver on the B200 engine (python/modisp/__init__.py:160-564).
 
@@ -343,16 +334,33 @@ class Solver:
         plugin.set_device(self.device)
         return "cuda", "B200 engine and sm_100 device available"
 
-    def _capacity(self, B, L, T, nmodes):
-        per_model = _workspace_per_model(L, T, nmodes)
+    def _capacity(self, B, L, T, nmodes, continuation=False):
+        """Models per chunk: as many of the B as the engine's workspace for them leaves within the
+        budget (workspace_bytes, else a quarter of the device's free memory)."""
+        o = _native.default_options()
+        o.single_precision, o.continuity_check = int(self.precision != "float64"), int(self.continuity_check)
+        o.continuation, o.log_points = int(continuation), int(self.tuning["log_points"] or 0)
+
+        def need(models):
+            return _native.workspace_bytes(models, L, T, nmodes, o)
+
+        n = max(1, min(B, self.chunk_size or B))
         if self.workspace_bytes is not None:
-            limit = max(1, int(self.workspace_bytes) // per_model)
-            if self.workspace_bytes < per_model:
+            budget = int(self.workspace_bytes)
+            if need(1) > budget:
                 raise MemoryError("workspace_bytes is too small for one model; increase the budget")
         else:
-            free, _ = _native.memory_info()
-            limit = max(1, int(0.4 * free) // per_model)
-        return max(1, min(B, limit, self.chunk_size or B))
+            budget = _native.memory_info()[0] // 4
+        if need(n) <= budget:
+            return n
+        fits = 1
+        while n - fits > 1:
+            mid = (fits + n) // 2
+            if need(mid) <= budget:
+                fits = mid
+            else:
+                n = mid
+        return fits
 
     def _key(self, L, T, nmodes, continuation):
         return (self.device, L, T, int(nmodes), self.accuracy, self.close_root_rtol, self.precision,
@@ -438,7 +446,7 @@ class Solver:
                 self._engine_key == (self._key(L, per.size, nmodes, continuation), B):
             capacity = B  # the engine of the last call fits: no look at the free memory
         else:
-            capacity = self._capacity(B, L, per.size, nmodes)
+            capacity = self._capacity(B, L, per.size, nmodes, continuation)
         engine, allocated = self._engine_for(capacity, L, per.size, nmodes, continuation)
         dtype = np.float32 if self.precision == "float32" else np.float64
         # the continuity screen runs in the FP32-scan engine (continuity_check)

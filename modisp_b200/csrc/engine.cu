@@ -242,10 +242,8 @@ int allow_shared(void (*kernel)(Args...), size_t bytes) {
   return 0;
 }
 
-int setup(md200_engine *e, bool staging) {
-  MD200_CK(cudaSetDevice(e->device));
-  MD200_CK(cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking));
-  MD200_CK(cudaStreamCreateWithFlags(&e->copy_stream, cudaStreamNonBlocking));
+// The engine's geometry and the workspace arrays for it, laid out but not allocated.
+int plan_workspace(md200_engine *e) {
   const int B = e->cap, L = e->L, T = e->T, nm = e->nmodes;
   Dev &d = e->d;
   d.Lmax = L;
@@ -317,7 +315,16 @@ int setup(md200_engine *e, bool staging) {
                     nt * nm * (2 * sizeof(double) + sizeof(unsigned)) + nt * 4 * sizeof(int) + nt +
                     md200_engine::MAX_CHUNKS * MD200_STAT_COUNT * sizeof(unsigned long long) +
                     2 * sizeof(double) * B + 64;
-  if (commit_plan(e)) return 1;
+  return 0;
+}
+
+int setup(md200_engine *e, bool staging) {
+  MD200_CK(cudaSetDevice(e->device));
+  MD200_CK(cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking));
+  MD200_CK(cudaStreamCreateWithFlags(&e->copy_stream, cudaStreamNonBlocking));
+  if (plan_workspace(e) || commit_plan(e)) return 1;
+  const Dev &d = e->d;
+  const int L = e->L;
   if (staging && need_staging(e)) return 1;
 
   // launch shapes
@@ -849,26 +856,34 @@ void md200_default_options(md200_options *o) {
   o->continuity_check = 1;
 }
 
+static int check_geometry(int capacity, int layers, int periods, int nmodes) {
+  if (capacity < 1 || layers < 1 || layers > 256 || periods < 1 || nmodes < 1 || nmodes > 256)
+    return fail("modisp_b200: invalid engine geometry (capacity >= 1, 1 <= layers <= 256, periods >= 1, "
+                "1 <= nmodes <= 256)");
+  return 0;
+}
+
+static void set_geometry(md200_engine *e, int capacity, int layers, int periods, int nmodes,
+                         const md200_options *options) {
+  e->cap = capacity;
+  e->L = layers;
+  e->T = periods;
+  e->nmodes = nmodes;
+  if (options) e->o = *options;
+  else md200_default_options(&e->o);
+}
+
 static md200_engine *create(int device, int capacity, int layers, int periods, int nmodes,
                             const md200_options *options, bool staging) {
   try {
-    if (capacity < 1 || layers < 1 || layers > 256 || periods < 1 || nmodes < 1 || nmodes > 256) {
-      fail("modisp_b200: invalid engine geometry (capacity >= 1, 1 <= layers <= 256, periods >= 1, "
-           "1 <= nmodes <= 256)");
-      return nullptr;
-    }
+    if (check_geometry(capacity, layers, periods, nmodes)) return nullptr;
     md200_engine *e = new (std::nothrow) md200_engine();
     if (!e) {
       fail("modisp_b200: out of host memory");
       return nullptr;
     }
     e->device = device;
-    e->cap = capacity;
-    e->L = layers;
-    e->T = periods;
-    e->nmodes = nmodes;
-    if (options) e->o = *options;
-    else md200_default_options(&e->o);
+    set_geometry(e, capacity, layers, periods, nmodes, options);
     bool failed = true;
     try {
       failed = setup(e, staging) != 0;
@@ -892,6 +907,18 @@ static md200_engine *create(int device, int capacity, int layers, int periods, i
 md200_engine *md200_create(int device, int capacity, int layers, int periods, int nmodes,
                            const md200_options *options) {
   return create(device, capacity, layers, periods, nmodes, options, true);
+}
+
+long long md200_workspace_bytes(int capacity, int layers, int periods, int nmodes, const md200_options *options) {
+  try {
+    if (check_geometry(capacity, layers, periods, nmodes)) return -1;
+    md200_engine e;
+    set_geometry(&e, capacity, layers, periods, nmodes, options);
+    return plan_workspace(&e) ? -1 : static_cast<long long>(e.plan_bytes);
+  } catch (...) {
+    fail_exception();
+    return -1;
+  }
 }
 
 md200_engine *md200_create_device(int device, int capacity, int layers, int periods, int nmodes,
