@@ -393,19 +393,25 @@ struct Ragged {
 // Runs of fewer traces list their brackets and roots as they come.
 constexpr int MODEL_LIST_MIN_TRACES = 4096;
 
-// Rounds of the split FP32 scan for a run of nt traces over an active set of
-// cap traces: enough for most traces to finish (a trace takes a round per
+// Rounds of the split FP32 scan for a run of nt traces of L rows over an active set
+// of cap traces: enough for most traces to finish (a trace takes a round per
 // SPLIT_SAMPLES samples and one per trough window, most take three); those still
 // unfinished after them are handed to the fused kernel.  A round of nothing costs
-// 35-40 us of launches, a handed-over trace a warp's scan of its rest.  Measured best
-// at 3, 120 and 1,200 thousand traces: 3 (Love) and 4 rounds (Rayleigh) per
-// active set; with nine, 120,000 Rayleigh traces took 4.41 ms against 4.16.  More
-// modes take a Rayleigh trace more rounds, and what the rounds leave costs the fused
-// kernel more: one round for every four brackets past seven (180,000 traces of ten
-// modes: 4 rounds 8.05 ms, 5 7.51, 9 7.6; 40,000 of a hundred modes: 4 14.6, 27 13.2).
-int split_rounds(int nt, int cap, int wave, int K) {
+// 35-90 us of launches, a handed-over trace a warp's scan of its rest.  With five
+// modes and fewer, 3 (Love) and 4 rounds (Rayleigh) per active set are best or within
+// 3 % of it from 30 thousand to 1.2 million traces.  More modes take a Rayleigh trace
+// more rounds: one for every four brackets past seven, to 27 (no trace needs more:
+// 300,000 traces of 256 modes 27.7 ms with 27, 30.1 with 63) -- where the traces
+// fill them.  Late rounds hold few traces, and a round pays from some hundred
+// thousand trace rows of the run on: a hundred modes, crustal models of 21 rows,
+// 17,400 traces 4 rounds 3.4 ms, 27 5.2; 42,000 traces 4 6.6, 9 6.3, 27 7.2; 150,000
+// traces 9 16.9, 27 15.2; 40,000 traces of up to 101 rows 4 14.6, 27 13.2.
+int split_rounds(int nt, int cap, int wave, int K, int L) {
   const int waves = (nt + cap - 1) / cap;
-  return std::min(md200_engine::MAX_SPLIT_ROUNDS, 3 * waves + (wave == 0 ? 1 + std::max(0, K - 7) / 4 : 0));
+  if (wave) return std::min(md200_engine::MAX_SPLIT_ROUNDS, 3 * waves);
+  const long long filled = static_cast<long long>(nt) * L / 100000 - 4;
+  const long long more = std::min<long long>({std::max(0, K - 7) / 4, 23, std::max(0LL, filled)});
+  return std::min(md200_engine::MAX_SPLIT_ROUNDS, 3 * waves + 1 + static_cast<int>(more));
 }
 
 // The split FP32 scan's launches (split_scan.cuh): `rounds` rounds, then the
@@ -534,7 +540,7 @@ int enqueue(md200_engine *e, const double *h, const double *vp, const double *vs
   const bool split = d.fp32 && (e->o.scan_mode == 2 ||
                                 (e->o.scan_mode == 0 && nt >= SPLIT_MIN_TRACES[wave]));
   if (split) {
-    const int rounds = split_rounds(nt, d.sp_cap, wave, d.K);
+    const int rounds = split_rounds(nt, d.sp_cap, wave, d.K, e->L);
     const int launched = wave == 0 ? split_scan<0>(e, dm, rounds, s) : split_scan<1>(e, dm, rounds, s);
     if (launched < 0) return fail("modisp_b200 CUDA: event record failed in the split scan");
     nl += launched;
