@@ -79,7 +79,7 @@ typedef struct md200_options {
                               search (<= 0: 2^22); an unfinished trace is re-scanned in FP64
                               with a limit of 2^26 (TRACE_ADAPTIVE_FALLBACK, level 24) */
   int scan_mode;           /* FP32 scan: 0 auto (rounds of split kernels for Rayleigh runs of
-                              16384 traces or more and Love runs of 131072, else the fused
+                              16384 traces or more and Love runs of 196608, else the fused
                               one-warp-per-trace kernel), 1 fused, 2 split; all return the
                               same brackets bit for bit */
 } md200_options;

@@ -8,7 +8,7 @@ forms of its scan, which put a different number of threads on a trace: the fused
 kernel (one warp per trace) and the split rounds (one thread per two samples for
 the values, one thread per trace for the bookkeeping, one warp per trace for the
 positions); the candidates cover both, and the automatic choice (split from 16,384
-Rayleigh or 131,072 Love traces on).  ``autotune`` times each candidate on a sample of the
+Rayleigh or 196,608 Love traces on).  ``autotune`` times each candidate on a sample of the
 caller's workload (device time of full runs, best of ``repeats``; both waves
 when ``wave`` is None), checks that every candidate returns bit-identical
 results (neither the launch shape nor the scan form may change a root), and

@@ -53,11 +53,13 @@ namespace md200 {
 constexpr int SPLIT_STEPS = 2;                    // 32-sample steps per trace per round
 constexpr int SPLIT_SAMPLES = 32 * SPLIT_STEPS;  // sample slots per active trace
 constexpr int SPLIT_ACTIVE_MAX = 1 << 20;         // active-set capacity (traces)
-// Runs with fewer traces use the fused kernel.  Scan stage, fused against split:
-// Rayleigh 9,000 traces 0.58 / 0.75 ms, 30,000 1.68 / 1.36, 120,000 6.65 / 4.16,
-// 1.2 million 78 / 37; Love, whose step is a tenth of the work, 30,000 0.50 / 0.65,
-// 120,000 1.91 / 1.97, 1.2 million 19.2 / 17.2.
-constexpr int SPLIT_MIN_TRACES[2] = {16384, 131072};
+// Runs with fewer traces use the fused kernel.  Scan stage, fused against split, five
+// modes: Rayleigh 9,000 traces 0.58 / 0.75 ms, 17,400 1.01 / 1.01, 24,000 1.37 / 1.24,
+// 150,000 8.2 / 5.0, 1.2 million 61 / 36; Love, whose step is a tenth of the work, 60,000
+// 0.96 / 1.11, 132,000 2.07 / 2.13, 198,000 3.08 / 3.03, 258,000 4.01 / 3.86, 1.2 million
+// 19.1 / 16.8.  With a hundred modes the lines lie somewhat higher for Love (132,000
+// 3.38 / 3.65, 198,000 5.05 / 5.23, 300,000 7.7 / 7.7) and are the same for Rayleigh.
+constexpr int SPLIT_MIN_TRACES[2] = {16384, 196608};
 constexpr unsigned SK_SEED = 1, SK_NEAR = 2, SK_EXACT = 4, SK_REDO = 8;
 constexpr int ZOOM_TROUGH = 0, ZOOM_LAST = 1;
 
