@@ -525,7 +525,9 @@ int enqueue(md200_engine *e, const double *h, const double *vp, const double *vs
   // traces refinement is latency-bound and the extra launches cost what it gains)
   Dev dm = d;
   dm.model_lists = nt >= MODEL_LIST_MIN_TRACES ? 1 : 0;
-  const int model_blocks = (B + 3) / 4;
+  auto list_grid = [&](int ranks) {
+    return static_cast<unsigned>((static_cast<long long>(B) * list_pieces(ranks, d.T) + 3) / 4);
+  };
   const auto refine_fn = wave == 0 ? refine<0> : refine<1>;
   // grids no larger than the run can fill: blocks with nothing to do cost a small
   // run more than its work (an empty pass of four kernels at full grids 27 us)
@@ -557,7 +559,7 @@ int enqueue(md200_engine *e, const double *h, const double *vp, const double *vs
   MD200_CK(cudaGetLastError());
   MD200_CK(mark(3));
   if (dm.model_lists) {
-    list_brackets<<<model_blocks, 128, 0, s>>>(d);
+    list_brackets<<<list_grid(d.K), 128, 0, s>>>(d);
     ++nl;
   }
   refine_fn<<<refine_blocks, 128, 0, s>>>(d);
@@ -590,7 +592,7 @@ int enqueue(md200_engine *e, const double *h, const double *vp, const double *vs
   MD200_CK(mark(8));
   if (d.group) {
     if (dm.model_lists) {
-      list_roots<<<model_blocks, 128, 0, s>>>(d);
+      list_roots<<<list_grid(d.nmodes), 128, 0, s>>>(d);
       ++nl;
     }
     group_velocity<<<group_blocks, 128, 0, s>>>(d);

@@ -1519,49 +1519,72 @@ __device__ __forceinline__ int brent_advance(BrentState &st, double tol, double 
 
 // ---------------------------------------------------------------------------
 // list_brackets, list_roots: the work of refine and group_velocity listed model by
-// model, and within a model by rank, then period; one warp per model.  Neighbours
-// in the list then share their layers, and their velocities vary smoothly, so the
-// lanes of a warp take the same branch of every layer's wave blocks and leave the
-// layer loop together.  (Appended trace by trace as the scan ends, a warp's 32
-// brackets came from five models and every rank: 17 of 32 lanes were active.)
-// Measured with settled guards (guard_settled), 20,000 low-velocity-layer models x
-// 60 periods, before -> after: refinement FP32-scan Rayleigh 17.5 -> 12.5 ms, FP64
-// Rayleigh 13.4 -> 10.6, FP32-scan Love 8.3 -> 5.6, FP64 Love 6.4 -> 4.9; group
-// velocity Rayleigh 3.01 -> 2.69, Love 1.37 -> 1.18; the listing itself 0.02 ms.
+// model, and within a model by rank, then period.  Neighbours in the list then share
+// their layers, and their velocities vary smoothly, so the lanes of a warp take the
+// same branch of every layer's wave blocks and leave the layer loop together.
+// (Appended trace by trace as the scan ends, a warp's 32 brackets came from five models
+// and every rank: 17 of 32 lanes were active.)  Measured with settled guards
+// (guard_settled), 20,000 low-velocity-layer models x 60 periods, before -> after:
+// refinement FP32-scan Rayleigh 17.5 -> 12.5 ms, FP64 Rayleigh 13.4 -> 10.6, FP32-scan
+// Love 8.3 -> 5.6, FP64 Love 6.4 -> 4.9; group velocity Rayleigh 3.01 -> 2.69, Love
+// 1.37 -> 1.18; the listing itself 0.02 ms.
+//
+// A warp lists one piece of a model, LIST_RANKS ranks of LIST_TRACES periods: with a
+// warp to a whole model, 256 modes of 70 models were a serial walk of 0.24 ms a list.
 // ---------------------------------------------------------------------------
+constexpr int LIST_RANKS = 8, LIST_TRACES = 64;
+__host__ __device__ constexpr int list_pieces(int ranks, int T) {
+  return ((ranks + LIST_RANKS - 1) / LIST_RANKS) * ((T + LIST_TRACES - 1) / LIST_TRACES);
+}
+
+// count(t, k0, k1, top): how many of trace t's ranks k0 .. k1 - 1 are taken, top raised
+// to one past the highest of them.
 template <class Count, class Take>
-__device__ __forceinline__ void list_by_model(const Dev &d, int *counter, int *list, Count count, Take take) {
-  const int lane = threadIdx.x & 31, b = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+__device__ __forceinline__ void list_by_model(const Dev &d, int ranks, int *counter, int *list, Count count,
+                                              Take take) {
+  const int lane = threadIdx.x & 31, piece = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int parts = (d.T + LIST_TRACES - 1) / LIST_TRACES, b = piece / list_pieces(ranks, d.T);
   if (b >= d.B || d.mstate[b] != 0) return;
+  const int of_model = piece - b * list_pieces(ranks, d.T);
+  const int k0 = of_model / parts * LIST_RANKS, k1 = min(k0 + LIST_RANKS, ranks);
+  const int f0 = of_model % parts * LIST_TRACES;
   const int first = d.ragged ? d.r_offsets[b] : b * d.T;
   const int traces = d.ragged ? d.r_offsets[b + 1] - first : d.T;
-  int total = 0, ranks = 0;
-  for (int f = lane; f < traces; f += 32) {
-    int most;
-    total += count(first + f, &most);
-    ranks = max(ranks, most);
-  }
+  // (a ragged model may have more periods than d.T: its parts go on in turn)
+  auto each = [&](auto body) {
+    for (int c = f0; c < traces; c += parts * LIST_TRACES)
+      for (int f = c; f < min(c + LIST_TRACES, traces); f += 32) body(first + f + lane, f + lane < traces);
+  };
+  int total = 0, top = k0;
+  each([&](int t, bool in) {
+    if (in) total += count(t, k0, k1, top);
+  });
   for (int o = 16; o; o >>= 1) {
     total += __shfl_xor_sync(FULL, total, o);
-    ranks = max(ranks, __shfl_xor_sync(FULL, ranks, o));
+    top = max(top, __shfl_xor_sync(FULL, top, o));
   }
+  if (!total) return;
   int at = 0;
-  if (lane == 0 && total) at = atomicAdd(counter, total);
+  if (lane == 0) at = atomicAdd(counter, total);
   at = __shfl_sync(FULL, at, 0);
-  for (int k = 0; k < ranks; ++k)
-    for (int f0 = 0; f0 < traces; f0 += 32) {
-      const int t = first + f0 + lane;
-      const bool take_it = f0 + lane < traces && take(t, k);
+  for (int k = k0; k < top; ++k)
+    each([&](int t, bool in) {
+      const bool take_it = in && take(t, k);
       const unsigned m = __ballot_sync(FULL, take_it);
       if (take_it) list[at + __popc(m & lanemask_lt())] = t * d.KB + k;
       at += __popc(m);
-    }
+    });
 }
 
 __global__ void __launch_bounds__(128) list_brackets(Dev d) {
   auto held = [&](int t) { return d.tflags[t] & TRACE_SEARCH_UNCONVERGED ? 0 : d.nbr[t]; };
   list_by_model(
-      d, &d.ctr[C_NREFINE], d.refine_list, [&](int t, int *most) { return *most = held(t); },
+      d, d.K, &d.ctr[C_NREFINE], d.refine_list,
+      [&](int t, int k0, int k1, int &top) {
+        const int end = min(held(t), k1);
+        top = max(top, end);
+        return max(0, end - k0);
+      },
       [&](int t, int k) { return k < held(t); });
 }
 
@@ -1571,11 +1594,14 @@ __global__ void __launch_bounds__(128) list_roots(Dev d) {
     return k < d.tr_modes[t] && d.gflags[static_cast<size_t>(d.tr_out[t]) + static_cast<size_t>(k) * d.tr_stride[t]] == 0;
   };
   list_by_model(
-      d, &d.ctr[C_NGROUP], d.group_list,
-      [&](int t, int *most) {
+      d, d.nmodes, &d.ctr[C_NGROUP], d.group_list,
+      [&](int t, int k0, int k1, int &top) {
         int n = 0;
-        for (int k = 0; k < d.tr_modes[t]; ++k) n += wanted(t, k);
-        *most = d.tr_modes[t];
+        for (int k = k0; k < k1; ++k)
+          if (wanted(t, k)) {
+            ++n;
+            top = max(top, k + 1);
+          }
         return n;
       },
       wanted);
