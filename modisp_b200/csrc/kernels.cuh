@@ -1872,8 +1872,12 @@ __global__ void assemble(Dev d, const int *list = nullptr, int count_id = 0) {
   }
   for (int i = 1; i < n; ++i)
     if (r(i) - r(i - 1) <= d.close_rtol * r(i)) fl |= TRACE_CLOSE_ROOT_RISK;
-  for (int mo = 0; mo < nm; ++mo) {
-    double root = mo < n ? r(mo) : NAN;
+  // (each root is read once, a mode ahead: read where the close-root test asks for them,
+  // its neighbours were two more waits a mode -- 60 traces of 256 modes 0.65 ms)
+  double below = NAN, c = n > 0 ? r(0) : NAN, above;
+  for (int mo = 0; mo < nm; ++mo, below = c, c = above) {
+    above = mo + 1 < n ? r(mo + 1) : NAN;
+    double root = c;
     if (isfinite(root) && root >= .99 * vs_hs) fl |= TRACE_NEAR_CUTOFF;
     if (isfinite(root) && d.accept < 1.) {
       double g, lm;
@@ -1891,9 +1895,7 @@ __global__ void assemble(Dev d, const int *list = nullptr, int count_id = 0) {
         d.gflags[cell] = GROUP_MISSING_ROOT;
       } else {
         // close-root test (cpp/cpu/solver.cpp:96-103)
-        const double c = r(mo);
-        const bool close = (mo && c - r(mo - 1) <= d.close_rtol * c) ||
-                           (mo + 1 < n && r(mo + 1) - c <= d.close_rtol * r(mo + 1));
+        const bool close = c - below <= d.close_rtol * c || above - c <= d.close_rtol * above;
         if (close) {
           d.grp[cell] = NAN;
           d.gflags[cell] = GROUP_CLOSE_ROOT;
