@@ -1408,44 +1408,19 @@ MD200_FN void love_multi(const LayerView<T> &m, const N *k, const N &w, N *F, N 
     ex[s] = 0;
     ev[s] = B(0);
   }
-  auto layer = [&](int j) {
+  for (int j = last - 1; j >= m.water; --j) {
     const T h = m.h(j), mu = m.rho(j) * m.vs2(j), imu = m.imu(j), ivs = m.ivs(j);
 #pragma unroll
     for (int s = 0; s < S; ++s) {
       const N kj = w * ivs;
       N cq, y, z;
-      if constexpr (sizeof(N) == sizeof(float)) {
-        // branch-free single precision: both forms, selected
-        N r, ir;
-        radical(k[s], kj, &r, &ir);
-        const float q = r * h;
-        float sn, cs;
-        m_sincos(q, &sn, &cs);
-        const float eq = m_exp(-q), f = eq * eq;
-        const bool prop = k[s] < kj;
-        cq = prop ? cs : .5f * (1.f + f);
-        const float half = prop ? sn : .5f * (1.f - f);
-        y = ir > 0.f ? half * ir : h;
-        z = prop ? -(r * half) : r * half;
-        ev[s] += prop ? 0.f : q;
-      } else {
-        ev[s] += love_entries<N, T>(k[s], kj, h, &cq, &y, &z);
-      }
+      ev[s] += love_entries<N, T>(k[s], kj, h, &cq, &y, &z);
       const N u = e[s][0] * cq + e[s][1] * z * mu;
       const N v = e[s][0] * y * imu + e[s][1] * cq;
       e[s][0] = u;
       e[s][1] = v;
       ex[s] += scale_vector(e[s], 2, tiny);
     }
-  };
-  if constexpr (sizeof(N) == sizeof(float)) {
-    // two layers per iteration: the next layer's special functions overlap this
-    // one's recurrence (measured 5 % faster for the FP32 Love scan, 9 % slower
-    // for the FP64 one, whose longer body already fills the pipes)
-#pragma unroll 2
-    for (int j = last - 1; j >= m.water; --j) layer(j);
-  } else {
-    for (int j = last - 1; j >= m.water; --j) layer(j);
   }
 #pragma unroll
   for (int s = 0; s < S; ++s) {
