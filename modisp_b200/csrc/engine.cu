@@ -1399,6 +1399,7 @@ int md200_kernel_report(int layers, int single_precision, char *json, int length
       {"scan_fp64_love", reinterpret_cast<const void *>(scan<double, 1>)},
       {"scan_fp32_love", reinterpret_cast<const void *>(scan<float, 1>)},
       {"refine", reinterpret_cast<const void *>(refine<0>)},
+      {"refine_love", reinterpret_cast<const void *>(refine<1>)},
       {"assemble", reinterpret_cast<const void *>(assemble)},
       {"group_velocity", reinterpret_cast<const void *>(group_velocity)},
   };
@@ -1414,7 +1415,7 @@ int md200_kernel_report(int layers, int single_precision, char *json, int length
     const int Ls = (layers + 3) & ~3;
     size_t dyn = 0;
     if (std::strncmp(en.name, "scan", 4) == 0)
-      dyn = scan_smem(4, Ls, std::strcmp(en.name, "scan_fp32") == 0 ? sizeof(float) : sizeof(double));
+      dyn = scan_smem(4, Ls, std::strncmp(en.name, "scan_fp32", 9) == 0 ? sizeof(float) : sizeof(double));
     int blocks = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, en.fn, 128, dyn);
     cudaGetLastError();
