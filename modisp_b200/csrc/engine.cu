@@ -171,8 +171,8 @@ int own_alloc(md200_engine *e, T **p, size_t count) {
 
 // setup()'s arrays come from one allocation: some fifty allocations and frees per
 // engine cost a call that makes its own engine (a ragged batch) more than its
-// solve.  1,000 models of 30-100 layers: 87 -> 34 ms a call, without the staging
-// below as well.
+// solve.  1,000 models of 30-100 layers: 86 -> 53 ms a call (up to a third less or
+// more from run to run), without the staging below as well.
 template <class T>
 int plan_alloc(md200_engine *e, T **p, size_t count) {
   *p = nullptr;
@@ -397,15 +397,16 @@ constexpr int MODEL_LIST_MIN_TRACES = 4096;
 // of cap traces: enough for most traces to finish (a trace takes a round per
 // SPLIT_SAMPLES samples and one per trough window, most take three); those still
 // unfinished after them are handed to the fused kernel.  A round of nothing costs
-// 35-90 us of launches, a handed-over trace a warp's scan of its rest.  With five
-// modes and fewer, 3 (Love) and 4 rounds (Rayleigh) per active set are best or within
-// 3 % of it from 30 thousand to 1.2 million traces.  More modes take a Rayleigh trace
-// more rounds: one for every four brackets past seven, to 27 (no trace needs more:
-// 300,000 traces of 256 modes 27.7 ms with 27, 30.1 with 63) -- where the traces
-// fill them.  Late rounds hold few traces, and a round pays from some hundred
-// thousand trace rows of the run on: a hundred modes, crustal models of 21 rows,
-// 17,400 traces 4 rounds 3.4 ms, 27 5.2; 42,000 traces 4 6.6, 9 6.3, 27 7.2; 150,000
-// traces 9 16.9, 27 15.2; 40,000 traces of up to 101 rows 4 14.6, 27 13.2.
+// 35-90 us of launches, a handed-over trace a warp's scan of its rest.  Rayleigh with
+// five modes: 4 rounds (7 over two active sets) are best or within 4 % of it from 24
+// thousand to 1.2 million traces.  Love: 3 rounds are, within 5 %, with 1 to 100 modes
+// and 130 to 600 thousand traces.  More modes take a Rayleigh trace more rounds: one
+// for every four brackets past seven, to 27 (no trace needs more: 300,000 traces of 256
+// modes 27.7 ms with 27, 30.1 with 63) -- where the traces fill them.  Late rounds hold
+// few traces, and a round pays from some hundred thousand trace rows of the run on: a
+// hundred modes, crustal models of 21 rows, 17,400 traces 4 rounds 3.4 ms, 27 5.2;
+// 42,000 traces 4 6.6, 9 6.3, 27 7.2; 150,000 traces 9 16.9, 27 15.2; 40,000 traces of
+// up to 101 rows 4 14.6, 27 13.2.
 int split_rounds(int nt, int cap, int wave, int K, int L) {
   const int waves = (nt + cap - 1) / cap;
   if (wave) return std::min(md200_engine::MAX_SPLIT_ROUNDS, 3 * waves);

@@ -17,8 +17,8 @@
 //                 point of the converged bracket
 //   [FP32 only] collect_repairs + scan<double>/refine on the traces whose
 //                 FP32 brackets FP64 did not confirm
-//   assemble      one thread per trace: order, cap and write the roots, flags,
-//                 counts and group-velocity windows
+//   assemble      one thread per trace: order, cap and write the roots, flags
+//                 and counts, mark the roots that get a group velocity
 //   group         one thread per root: FP64 group velocity from forward-mode
 //                 derivatives dF/dk and dF/domega of the secular function
 //   [FP32 only] continuity_screen + scan<double>/refine/assemble/group on the

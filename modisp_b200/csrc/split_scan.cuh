@@ -225,7 +225,6 @@ __device__ __forceinline__ bool split_near(const Dev &d, int t, SplitRound &smp,
 // single evaluation the fused scan makes).  A slot past the
 // window or in the near-cutoff band leaves its half to a copy of the other
 // sample, whose result is not stored.
-static_assert(SPLIT_SAMPLES == 64, "the paired evaluation takes the two 32-sample steps of a round");
 //
 // A warp takes one trace's 32 pairs after another.  The layer records of the next
 // trace's model come into shared memory (cp.async) while the current trace is
@@ -236,6 +235,7 @@ static_assert(SPLIT_SAMPLES == 64, "the paired evaluation takes the two 32-sampl
 // fewer instructions, FMA pipe 67 % busy; the FMA pipe's own time is 15 ms).
 // Dynamic shared memory: `buffers` (2, or 1 where two would cost resident CTAs)
 // x Ls records for each of the 4 warps.
+static_assert(SPLIT_SAMPLES == 64, "the paired evaluation takes the two 32-sample steps of a round");
 inline size_t split_pair_smem(int wave, int Ls, int buffers) {
   return static_cast<size_t>(4) * buffers * Ls * pair_row(wave) * 2 * sizeof(float);
 }
